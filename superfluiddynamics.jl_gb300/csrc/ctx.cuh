@@ -173,6 +173,16 @@ static int upload_dw(gpss_ctx *c, void **dev, const std::vector<ldouble> &re, co
     return GPSS_OK;
 }
 
+// fixed-point table entries (the register passes of FP64 fields)
+static int upload_fx(gpss_ctx *c, void **dev, const std::vector<int4> &t)
+{
+    GPSS_TRY(dev_alloc(c, dev, t.size() * sizeof(int4)));
+    CUDA_TRY(c, cudaMemcpy(*dev, t.data(), t.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    return GPSS_OK;
+}
+// does this axis run the register pass of an FP64 field (fixed-point tables)?
+static bool fx_axis(const gpss_ctx *c, int axis) { return c->precision == GPSS_FP64 && !c->gen[axis]; }
+
 static void clear_graphs(gpss_ctx *c);
 
 // Kinetic factor table for `axis` (splitting.jl:167/172/190/195/200):
@@ -196,7 +206,9 @@ static int get_phase(gpss_ctx *c, int axis, double dtl, int imag, int fused, con
     const bool rot = c->omega != 0.0 && axis < 2 && c->ndim >= 2;
     const int64_t rows = rot ? (axis == 0 ? c->n[1] : c->n[0]) : 1;
     std::vector<ldouble> re((size_t)(n * rows)), im((size_t)(n * rows));
-    const ldouble inv_n = fused ? 1.0L / (ldouble)n : 1.0L;
+    // fixed-point passes divide by n (a power of two) on the way out
+    const bool fx = fused && fx_axis(c, axis);
+    const ldouble inv_n = fused && !fx ? 1.0L / (ldouble)n : 1.0L;
     for (int64_t r = 0; r < rows; r++) {
         const double cr = rot ? (axis == 0 ? c->coord[1][(size_t)r] : c->coord[0][(size_t)r]) : 0.0;
         for (int64_t k = 0; k < n; k++) {
@@ -215,8 +227,9 @@ static int get_phase(gpss_ctx *c, int axis, double dtl, int imag, int fused, con
             im[(size_t)(r * n + k)] = fi * inv_n;
         }
     }
-    PhaseEntry e{axis, imag, fused, dtl, c->cD, c->omega, nullptr, rot ? 2 * n : 0};
-    GPSS_TRY(upload_dw(c, &e.dev, re, im, rows, n));
+    PhaseEntry e{axis, imag, fused, dtl, c->cD, c->omega, nullptr, rot ? (fx ? n : 2 * n) : 0};
+    if (fx) GPSS_TRY(upload_fx(c, &e.dev, fx_phase_table(re, im)));
+    else GPSS_TRY(upload_dw(c, &e.dev, re, im, rows, n));
     if (c->phases.size() > 64) {  // bounded cache: drop the oldest
         clear_graphs(c);
         cudaStreamSynchronize(c->stream);
@@ -340,9 +353,11 @@ template <typename T> static int blocks_for(gpss_ctx *c, int axis)
 // while a y/z tile takes n row copies of 128 bytes, which the copy engine
 // moves about 3x slower than coalesced loads; at 256^3 the direct kernel's x
 // pass is also 6% faster than the pipelined one (issue-bound, more warps).
+// FP32 only: the passes of FP64 fields are bound by their arithmetic, and the
+// direct kernel runs it in fixed point.
 static bool pipe_ok(const gpss_ctx *c, int axis)
 {
-    if (!(c->flags & GPSS_FLAG_PIPE)) return false;
+    if (!(c->flags & GPSS_FLAG_PIPE) || c->precision != GPSS_FP32) return false;
     if (axis != 0) return false;
     const int64_t n = c->n[axis];
     if (n != 64 && n != 128 && n != 256) return false;

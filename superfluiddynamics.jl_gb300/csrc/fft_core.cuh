@@ -10,7 +10,9 @@
 // output in natural frequency order in a[0..N).  With full unrolling the
 // reordering is register renaming only.
 #pragma once
+#include <type_traits>
 #include <cuda_runtime.h>
+#include "fft_fix.cuh"
 
 namespace gpss {
 
@@ -139,6 +141,8 @@ template <typename T> __device__ __forceinline__ T rmul2(T t, T hi, T lo) { retu
 template <int M, int DIR, typename V> __device__ __forceinline__ V mul_w16(V a)
 {
     using T = decltype(V::x);
+    if constexpr (std::is_integral<T>::value) return fx_mul_w16<M, DIR>(a);  // fixed point (FP64 fields)
+    else {
     using K = DftConst<T>;
     constexpr int m = ((M % 16) + 16) % 16;
     constexpr bool packed = GPSS_PACKED_DFT && sizeof(T) == 4;
@@ -177,6 +181,7 @@ template <int M, int DIR, typename V> __device__ __forceinline__ V mul_w16(V a)
         const T srh = (si == 2 || si == -2) ? (T)(si > 0 ? K::S1h : -K::S1h) : (T)(si > 0 ? K::C1h : -K::C1h);
         const T srl = (si == 2 || si == -2) ? (T)(si > 0 ? K::S1l : -K::S1l) : (T)(si > 0 ? K::C1l : -K::C1l);
         return cmul2(a, mk<V>(crh, (T)DIR * srh), mk<V>(crl, (T)DIR * srl));
+    }
     }
 }
 

@@ -1,0 +1,244 @@
+// fft_fix.cuh -- FP64 fields transformed in 64-bit fixed point.
+//
+// GB300 runs FP64 at 2 operations per clock and SM, 32-bit integer additions at
+// 128 and 32x32 -> 64-bit multiply-adds at ~24 (measured).  A transform in
+// FP64 arithmetic is bound by that pipe alone (72 operations per cell and
+// pass of 256-cell lines: 2.5 ms at 256^3, against 0.08 ms of memory traffic),
+// so the passes of FP64 fields hold the values of a line as 64-bit integers
+// on a common quantum: a complex addition is four 32-bit additions, a product
+// by a constant of 63 bits twelve multiply-adds.
+//
+// Accuracy and range.  The quantum of a line comes from its 2-norm: with
+// ||x|| <= 2^E a value is an integer multiple of 2^(E - 60), rounded to nearest
+// on entry.  A sum of m of the line's values is at most sqrt(m) ||x||, a
+// transform of n cells multiplies the norm by sqrt(n), the phase (modulus at
+// most 1) does not raise it, and each product by a table constant (2^62 times
+// its value, used as a 2^64 one) divides by 4.  So for n <= 256 = 16 x 16 every
+// stage holds at most 4 ||x|| = 2^62 in modulus: sqrt(16) after stage A,
+// sqrt(256) / 4 after stage B, sqrt(16 256) / 16 after its backward part,
+// 256 / 64 at the end; shorter lines stay below.  The quantum of each stage
+// grows like the values do, so every rounding on the way is about 2^-57 of the
+// line's rms (n = 256; smaller for shorter lines) whatever its shape, and the
+// result is rounded once to FP64 (2^-53 of itself): closer to the exact pass
+// than FP64 arithmetic, whose every operation rounds at 2^-53
+// (tests/test_gpu_fixed_point.py holds it to that).
+//
+// A line that holds NaN or infinity (or a component of 2^1017 and above,
+// whose square is infinite anyway) comes out as NaN throughout, as a sum over
+// it would.
+#pragma once
+#include <cstdint>
+#include <cuda_runtime.h>
+
+namespace gpss {
+
+// a complex value in fixed point
+struct __align__(16) fxc {
+    long long x, y;
+};
+
+__device__ __forceinline__ long long fx_madw(int a, int b, long long c)
+{
+    long long d;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+    return d;
+}
+// a = h 2^32 + l with both halves signed, so that signed multiply-adds serve
+// every partial product
+__device__ __forceinline__ void fx_split(long long a, int &h, int &l)
+{
+    l = (int)a;
+    h = (int)(a >> 32) + (int)((unsigned)l >> 31);
+}
+// A product's partial sums: S in units of 2^64 / 2^64, X in units of 2^32 / 2^64
+// of the result.  X starts at one half (rounding) plus 2^63, which keeps it
+// unsigned so that its upper half adds without a sign extension; S starts at
+// minus that offset.  The low-by-low product (below the rounding) is left out;
+// with signed halves its mean is zero.
+constexpr long long FX_S0 = -(1LL << 31);
+constexpr long long FX_X0 = (long long)((1ULL << 63) + (1ULL << 31));
+__device__ __forceinline__ long long fx_fold(long long S, long long X)
+{
+    return S + (long long)((unsigned long long)X >> 32);
+}
+// a (rh 2^32 + rl) 2^-64
+__device__ __forceinline__ long long fx_rmul(long long a, int rh, int rl)
+{
+    int h, l;
+    fx_split(a, h, l);
+    return fx_fold(fx_madw(h, rh, FX_S0), fx_madw(l, rh, fx_madw(h, rl, FX_X0)));
+}
+
+// A table constant: 2^62 times a complex number of modulus at most 1, the
+// halves of each component signed (c = h 2^32 + l).
+// a * c / 4 and a * conj(c) / 4
+template <bool CONJ> __device__ __forceinline__ fxc fx_cmul(fxc a, int4 c)
+{
+    int xh, xl, yh, yl;
+    fx_split(a.x, xh, xl);
+    fx_split(a.y, yh, yl);
+    const int rl = c.x, rh = c.y;
+    const int pl = CONJ ? -c.z : c.z, ph = CONJ ? -c.w : c.w;    // imaginary part
+    const int ml = CONJ ? c.z : -c.z, mh = CONJ ? c.w : -c.w;    // minus it
+    fxc o;
+    o.x = fx_fold(fx_madw(xh, rh, fx_madw(yh, mh, FX_S0)),
+                  fx_madw(xl, rh, fx_madw(yl, mh, fx_madw(xh, rl, fx_madw(yh, ml, FX_X0)))));
+    o.y = fx_fold(fx_madw(yh, rh, fx_madw(xh, ph, FX_S0)),
+                  fx_madw(yl, rh, fx_madw(xl, ph, fx_madw(yh, rl, fx_madw(xh, pl, FX_X0)))));
+    return o;
+}
+// a / 4, rounded: what a product by the constant 1 gives
+__device__ __forceinline__ fxc fx_quarter(fxc a)
+{
+    return fxc{(a.x + 2) >> 2, (a.y + 2) >> 2};
+}
+
+// the DFT-16's own constants as 2^64 times a number below 1/2, signed halves
+constexpr long long FX_TAN16 = 0x32ebebc0aa62b00fLL;   // tan(pi/16)
+constexpr long long FX_SIN8 = 0x61f78a9abaa58b47LL;    // sin(pi/8)
+constexpr long long FX_1MH = 0x4afb0ccc06219b7cLL;     // 1 - sqrt(1/2)
+__host__ __device__ constexpr int fx_lo(long long c) { return (int)(unsigned)(c & 0xffffffffLL); }
+__host__ __device__ constexpr int fx_hi(long long c) { return (int)((c - (long long)fx_lo(c)) >> 32); }
+
+// rotation by D pi/8 (D = +-1) in three shears (Buneman's lifting form of a
+// plane rotation): 9 multiply-adds instead of 12
+template <int D> __device__ __forceinline__ fxc fx_rot8(fxc a)
+{
+    constexpr int th = -D * fx_hi(FX_TAN16), tl = -D * fx_lo(FX_TAN16);
+    constexpr int sh = D * fx_hi(FX_SIN8), sl = D * fx_lo(FX_SIN8);
+    a.x += fx_rmul(a.y, th, tl);
+    a.y += fx_rmul(a.x, sh, sl);
+    a.x += fx_rmul(a.y, th, tl);
+    return a;
+}
+// a sqrt(1/2)
+__device__ __forceinline__ long long fx_half_sqrt(long long a)
+{
+    return a + fx_rmul(a, -fx_hi(FX_1MH), -fx_lo(FX_1MH));
+}
+
+// a * exp(DIR 2 pi i M / 16)
+template <int M, int DIR> __device__ __forceinline__ fxc fx_mul_w16(fxc a)
+{
+    constexpr int m = (((DIR * M) % 16) + 16) % 16;  // exp(2 pi i m / 16)
+    if constexpr (m == 0) return a;
+    else if constexpr (m == 4) return fxc{-a.y, a.x};
+    else if constexpr (m == 8) return fxc{-a.x, -a.y};
+    else if constexpr (m == 12) return fxc{a.y, -a.x};
+    else if constexpr (m % 2 == 0) {
+        // (sc + i ss) / sqrt 2
+        constexpr int sc = (m == 2 || m == 14) ? 1 : -1, ss = (m == 2 || m == 6) ? 1 : -1;
+        const long long u = ss > 0 ? a.x - a.y : a.x + a.y;  // sc x - ss y, up to sc when sc ss > 0 ...
+        const long long v = ss > 0 ? a.x + a.y : a.y - a.x;
+        // (x + i y)(sc + i ss) = (sc x - ss y) + i (ss x + sc y)
+        if constexpr (sc > 0) return fxc{fx_half_sqrt(u), fx_half_sqrt(v)};
+        else if constexpr (ss > 0) return fxc{-fx_half_sqrt(v), fx_half_sqrt(u)};   // m = 6: -(x + y), x - y
+        else return fxc{fx_half_sqrt(a.y - a.x), -fx_half_sqrt(a.x + a.y)};          // m = 10
+    } else if constexpr (m == 1) return fx_rot8<1>(a);
+    else if constexpr (m == 15) return fx_rot8<-1>(a);
+    else if constexpr (m == 3) { const fxc b = fx_rot8<-1>(a); return fxc{-b.y, b.x}; }
+    else if constexpr (m == 5) { const fxc b = fx_rot8<1>(a); return fxc{-b.y, b.x}; }
+    else if constexpr (m == 7) { const fxc b = fx_rot8<-1>(a); return fxc{-b.x, -b.y}; }
+    else if constexpr (m == 9) { const fxc b = fx_rot8<1>(a); return fxc{-b.x, -b.y}; }
+    else if constexpr (m == 11) { const fxc b = fx_rot8<-1>(a); return fxc{b.y, -b.x}; }
+    else { const fxc b = fx_rot8<1>(a); return fxc{b.y, -b.x}; }  // m = 13
+}
+
+// log2 of a line length
+template <int N> struct FxLog { static constexpr int V = 1 + FxLog<N / 2>::V; };
+template <> struct FxLog<1> { static constexpr int V = 0; };
+
+// The largest upper word of the magnitudes of n values' components.  Upper
+// words of non-negative doubles order like floats, and a float maximum takes
+// the absolute value for free; NaN-propagating, so that words that look like a
+// float NaN (2^1017 and above) win.
+template <int N> __device__ __forceinline__ int fx_max_word(const double2 *v)
+{
+    float m = 0.f;
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        const float a = fabsf(__int_as_float(__double2hiint(v[j].x)));
+        const float b = fabsf(__int_as_float(__double2hiint(v[j].y)));
+        asm("max.NaN.f32 %0, %0, %1;" : "+f"(m) : "f"(a));
+        asm("max.NaN.f32 %0, %0, %1;" : "+f"(m) : "f"(b));
+    }
+    return __float_as_int(m);
+}
+// the biased exponent that sums of squares are taken relative to
+__device__ __forceinline__ int fx_ref(int word) { return max(word >> 20, 64); }
+// sum of the squares of n values over 2^(2 (ref - 1023)), ref at least the
+// exponent of each: an upper word becomes the float of the same significand by
+// a shift and an offset (components below 2^-100 of the reference count as that)
+template <int N> __device__ __forceinline__ float fx_norm2(const double2 *v, int ref)
+{
+    const float low = __int_as_float(max(ref - 100, 0) << 20);
+    const int off = 0x3f800000 - (int)((unsigned)ref << 23);
+    float s = 0.f;
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        const float a = __int_as_float((int)((unsigned)__float_as_int(fmaxf(
+            fabsf(__int_as_float(__double2hiint(v[j].x))), low)) << 3) + off);
+        const float b = __int_as_float((int)((unsigned)__float_as_int(fmaxf(
+            fabsf(__int_as_float(__double2hiint(v[j].y))), low)) << 3) + off);
+        s = fmaf(a, a, fmaf(b, b, s));
+    }
+    return s;
+}
+// log2 of the quantum of a line: its 2-norm is sqrt(s) 2^(ref - 1023), at most
+// 2^(q + 60) (s, of truncated significands, is short of the true sum by less
+// than 2^-18 of it, and sqrt(1 + 2^-18) is within the bounds' own slack)
+__device__ __forceinline__ int fx_quantum(int ref, float s)
+{
+    const int es = (__float_as_int(s) >> 23) - 127;  // s < 2^(es + 1)
+    return max(ref - 1023 + ((es + 2) >> 1) - 60, -1020);
+}
+
+// x on the quantum 2^q, rounded to nearest: s0 = 1084 + q.  The significand, left-justified below the sign bit, is
+// shifted to half the quantum, given its sign, and rounded up by one half.
+__device__ __forceinline__ long long fx_from(double x, int s0)
+{
+    const int hi = __double2hiint(x);
+    const unsigned lo = (unsigned)__double2loint(x);
+    const int s = min(s0 - ((hi >> 20) & 0x7ff), 63);  // 0 and denormals: to 0
+    const unsigned mh = (__funnelshift_l(lo, (unsigned)hi, 10) & 0x3fffffffu) | 0x40000000u;
+    const unsigned long long m = ((unsigned long long)mh << 32) | (unsigned long long)(lo << 10);
+    const long long sg = (long long)(hi >> 31);
+    return ((((long long)(m >> s)) ^ sg) - sg + 1) >> 1;
+}
+
+// Leaving fixed point: an integer v times 2^q as the FP64 nearest to it.  The
+// halves of v are placed in the significands of 2^84 2^q and 2^52 2^q, so two
+// additions (the first exact) give the value; q outside the range that their
+// exponents leave is applied as a second factor.
+struct FxOut {
+    int hw, lw;
+    double k, f;
+    bool scaled;
+    __device__ __forceinline__ FxOut(int q, bool bad, double scale, bool with_scale)
+    {
+        const int qc = min(max(q, -1000), 900), d = min(max(q - qc, -1000), 1000);
+        hw = 0x45300000 + qc * (1 << 20);
+        lw = 0x43300000 + qc * (1 << 20);
+        k = bad ? __longlong_as_double(0x7ff8000000000000LL)
+                : __hiloint2double(0x45300000 + qc * (1 << 20), (int)0x80100000);
+        scaled = with_scale || d != 0;
+        f = __hiloint2double((1023 + d) << 20, 0) * scale;
+    }
+    __device__ __forceinline__ double real(long long v) const
+    {
+        const double h = __hiloint2double(hw, (int)((unsigned)(v >> 32) ^ 0x80000000u));
+        const double l = __hiloint2double(lw, (int)v);
+        return (h - k) + l;
+    }
+    __device__ __forceinline__ double2 operator()(fxc c) const
+    {
+        double2 o = make_double2(real(c.x), real(c.y));
+        if (scaled) {
+            o.x *= f;
+            o.y *= f;
+        }
+        return o;
+    }
+};
+
+}  // namespace gpss

@@ -484,7 +484,9 @@ int gpss_create(gpss_ctx **out, int ndim, const int64_t *n, const double *lo, co
         } else {
             // two rows: stage-A order (k1*N2 + r) and stage-B order (r*N1 + k1)
             twiddle_rows(na, re, im);
-            if ((rc = upload_dw(c, &c->tw[a], re, im, 2, na))) return bail(rc);
+            if ((rc = fx_axis(c, a) ? upload_fx(c, &c->tw[a], fx_table(re, im))
+                                    : upload_dw(c, &c->tw[a], re, im, 2, na)))
+                return bail(rc);
         }
         if ((rc = dev_alloc(c, (void **)&c->coord_dev[a], sizeof(double) * (size_t)c->n[a]))) return bail(rc);
         e = cudaMemcpy(c->coord_dev[a], c->coord[a].data(), sizeof(double) * (size_t)c->n[a], cudaMemcpyHostToDevice);

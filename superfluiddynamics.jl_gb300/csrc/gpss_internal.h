@@ -77,6 +77,56 @@ std::vector<vec2<T>> dw_split(const std::vector<long double> &re, const std::vec
     return out;
 }
 
+// One component of a fixed-point table constant (fft_fix.cuh): 2^62 v for
+// |v| <= 1 as halves h 2^32 + l, both signed.  l = -2^31 has no negative, so
+// it moves by one unit of 2^-62.
+inline void fx_halves(long double v, int &l, int &h)
+{
+    int64_t c = (int64_t)llroundl(v * 4611686018427387904.0L);
+    if ((uint32_t)c == 0x80000000u) c += c < 0 ? -1 : 1;
+    l = (int)(uint32_t)c;
+    h = (int)((c - (int64_t)l) >> 32);
+}
+inline int4 fx_const(long double re, long double im)
+{
+    int4 c;
+    fx_halves(re, c.x, c.y);
+    fx_halves(im, c.z, c.w);
+    return c;
+}
+// Constants of modulus at most 1 in fixed point.
+inline std::vector<int4> fx_table(const std::vector<long double> &re, const std::vector<long double> &im)
+{
+    std::vector<int4> t(re.size());
+    for (size_t i = 0; i < t.size(); i++) t[i] = fx_const(re[i], im[i]);
+    return t;
+}
+// A fixed-point phase or multiplier table: a leading entry with the exponent e,
+// then the values divided by 2^e, the smallest power of two at or above their
+// largest modulus.  A non-finite value makes every result of a pass with the
+// table NaN or infinite in FP64; here its exponent overflows the pass's result.
+inline std::vector<int4> fx_phase_table(const std::vector<long double> &re, const std::vector<long double> &im)
+{
+    long double m = 0.0L;
+    bool finite = true;
+    for (size_t i = 0; i < re.size(); i++) {
+        const long double a = hypotl(re[i], im[i]);
+        finite = finite && std::isfinite((double)a);
+        if (a > m) m = a;
+    }
+    int e = 0;
+    if (finite && m > 0.0L) {
+        const long double f = frexpl(m, &e);  // m = f 2^e, f in [1/2, 1)
+        // unit moduli are 1 up to the rounding of the long double values
+        if (f <= 0.5L * (1.0L + 1e-17L)) e--;
+    }
+    std::vector<int4> t(re.size() + 1);
+    t[0] = make_int4(finite ? e : 1 << 20, 0, 0, 0);
+    for (size_t i = 0; i < re.size(); i++)
+        t[i + 1] = finite ? fx_const(ldexpl(re[i], -e), ldexpl(im[i], -e)) : fx_const(1.0L, 0.0L);
+    return t;
+}
+
 // pass launchers (pass_f32.cu / pass_f64.cu)
 cudaError_t launch_pass_f32(int mode, bool xl, int n, const PassArgs<float> &a, int blocks,
                             cudaStream_t s);
@@ -84,9 +134,8 @@ cudaError_t launch_pass_f64(int mode, bool xl, int n, const PassArgs<double> &a,
                             cudaStream_t s);
 int pass_lines_per_cta_f32(int n, bool xl);
 int pass_lines_per_cta_f64(int n, bool xl);
-// pipelined fused pass (n in {64, 128, 256}; tiles of 4096/n lines)
+// pipelined fused pass (FP32; n in {64, 128, 256}; tiles of 4096/n lines)
 cudaError_t launch_pipe_f32(bool xl, int n, const PassArgs<float> &a, int ntiles, cudaStream_t s);
-cudaError_t launch_pipe_f64(bool xl, int n, const PassArgs<double> &a, int ntiles, cudaStream_t s);
 
 // the generic-length pass (pass_gen.cu)
 cudaError_t launch_gen_f32(int mode, const PassArgs<float> &a, const GenPlan &p, cudaStream_t s);
@@ -110,10 +159,7 @@ template <> struct PassLauncher<double> {
     static cudaError_t launch(int mode, bool xl, int n, const PassArgs<double> &a, int blocks,
                               cudaStream_t s) { return launch_pass_f64(mode, xl, n, a, blocks, s); }
     static int lines(int n, bool xl) { return pass_lines_per_cta_f64(n, xl); }
-    static cudaError_t pipe(bool xl, int n, const PassArgs<double> &a, int ntiles, cudaStream_t s)
-    {
-        return launch_pipe_f64(xl, n, a, ntiles, s);
-    }
+    static cudaError_t pipe(bool, int, const PassArgs<double> &, int, cudaStream_t) { return cudaErrorInvalidValue; }
     static cudaError_t gen(int mode, const PassArgs<double> &a, const GenPlan &p, cudaStream_t s)
     {
         return launch_gen_f64(mode, a, p, s);

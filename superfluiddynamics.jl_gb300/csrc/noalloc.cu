@@ -51,9 +51,8 @@ constexpr size_t kOffPartials = kOffTw + 3 * 4 * 256 * 16;         // RQ_COUNT x
 constexpr size_t kPartialBytes = GPSS_NOALLOC_SCRATCH_BYTES - kOffPartials;
 
 // The largest field the entry point takes (256^3) has at most 256^2 / W
-// tiles in one pass, W the lines of a CTA (fewest for the FP64 passes: 4), so
-// its partial sums need 16384 x 5 doubles = 640 KiB of the 969.5 KiB region
-// (1.5x margin).  The run-time check below therefore never rejects a field of
+// tiles in one pass, W the lines of a CTA (fewest: 8), so its partial sums
+// need 8192 x 5 doubles = 320 KiB of the 969.5 KiB region (3x margin).  The run-time check below therefore never rejects a field of
 // lines up to 256; it guards the limit should the CTA shapes change.
 static_assert((uint64_t)(256 * 256 / PassShape<double, 256, true>::W) * RQ_COUNT * sizeof(double) <=
                   kPartialBytes, "the partial sums of a 256^3 FP64 field must fit the scratch array");
@@ -79,13 +78,18 @@ int noalloc_fail(int code, const char *msg, cudaError_t e = cudaSuccess)
     return gpss::fail(nullptr, code, "gpss_energy_noalloc: %s", msg);
 }
 
-// twiddle tables of one axis in the pass kernel's layout (stage A hi, lo;
-// stage B hi, lo)
-template <typename T> std::vector<vec2<T>> twiddle_table(int64_t n)
+// twiddle tables of one axis in the pass kernel's layout, as bytes (FP32: stage
+// A hi, lo; stage B hi, lo; FP64: fixed point, stage A, stage B)
+template <typename T> std::vector<unsigned char> twiddle_table(int64_t n)
 {
     std::vector<long double> re, im;
     twiddle_rows(n, re, im);
-    return dw_split<T>(re, im, n);
+    auto bytes = [](const auto &t) {
+        const unsigned char *p = reinterpret_cast<const unsigned char *>(t.data());
+        return std::vector<unsigned char>(p, p + t.size() * sizeof(t[0]));
+    };
+    if constexpr (sizeof(T) == 8) return bytes(fx_table(re, im));
+    else return bytes(dw_split<T>(re, im, n));
 }
 
 double lerp_node(int64_t j, int64_t d, double a, double b)
@@ -118,9 +122,9 @@ int energy_noalloc_t(int ndim, const int64_t *n3, const double *lo, const double
         e = cudaMemcpyAsync(coord + 256 * a, x.data(), sizeof(double) * (size_t)n3[a], cudaMemcpyHostToDevice,
                             stream);
         if (e != cudaSuccess) return noalloc_fail(GPSS_ECUDA, "cudaMemcpyAsync (coordinates)", e);
-        const std::vector<vec2<T>> t = twiddle_table<T>(n3[a]);
-        e = cudaMemcpyAsync(tw + (size_t)a * 4 * 256 * sizeof(vec2<T>), t.data(), sizeof(vec2<T>) * t.size(),
-                            cudaMemcpyHostToDevice, stream);
+        const std::vector<unsigned char> t = twiddle_table<T>(n3[a]);
+        e = cudaMemcpyAsync(tw + (size_t)a * 4 * 256 * sizeof(vec2<T>), t.data(), t.size(), cudaMemcpyHostToDevice,
+                            stream);
         if (e != cudaSuccess) return noalloc_fail(GPSS_ECUDA, "cudaMemcpyAsync (twiddles)", e);
     }
     const int64_t nx = n3[0], ny = n3[1];
@@ -193,9 +197,8 @@ extern "C" int gpss_energy_noalloc(int ndim, const int64_t *n, const double *lo,
     }
     // the partial sums of the largest pass must fit the fixed scratch, counted
     // from the tile count (an upper bound on the grid, which may be capped at
-    // one wave).  The largest accepted field, 256^3 in FP64 (64-thread CTAs,
-    // 4 lines each: 16384 tiles x 5 sums x 8 B = 640 KiB), fits with a 1.6x
-    // margin, so today this refusal is a guard for changed launch shapes.
+    // one wave).  The largest accepted field, 256^3 (CTAs of 8 lines: 8192
+    // tiles x 5 sums x 8 B = 320 KiB), fits with a 3x margin, so today this refusal is a guard for changed launch shapes.
     const int64_t total = n3[0] * n3[1] * n3[2];
     for (int a = 0; a < ndim; a++) {
         const int W = precision == GPSS_FP32 ? pass_lines_per_cta_f32((int)n3[a], a == 0)

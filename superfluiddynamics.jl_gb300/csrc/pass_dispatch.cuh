@@ -212,10 +212,7 @@ template <typename T, int N> static int lines_per_cta_n(bool xl)
         return launch_pass_n<T, N>(mode, xl, a, blocks, s);                                    \
     }
 
-#define GPSS_DEFINE_PASS_DISPATCH(T, SUFFIX)                                                   \
-    GPSS_DECLARE_PASS_N(T, SUFFIX, 64)                                                         \
-    GPSS_DECLARE_PASS_N(T, SUFFIX, 128)                                                        \
-    GPSS_DECLARE_PASS_N(T, SUFFIX, 256)                                                        \
+#define GPSS_DEFINE_PIPE_DISPATCH(T, SUFFIX)                                                   \
     cudaError_t launch_pipe_##SUFFIX(bool xl, int n, const PassArgs<T> &a, int ntiles,         \
                                      cudaStream_t s)                                           \
     {                                                                                          \
@@ -228,7 +225,12 @@ template <typename T, int N> static int lines_per_cta_n(bool xl)
                             : launch_pipe_inst<T, 256, false>(a, ntiles, s);                   \
         default: return cudaErrorInvalidValue;                                                 \
         }                                                                                      \
-    }                                                                                          \
+    }
+
+#define GPSS_DEFINE_PASS_DISPATCH(T, SUFFIX)                                                   \
+    GPSS_DECLARE_PASS_N(T, SUFFIX, 64)                                                         \
+    GPSS_DECLARE_PASS_N(T, SUFFIX, 128)                                                        \
+    GPSS_DECLARE_PASS_N(T, SUFFIX, 256)                                                        \
     cudaError_t launch_pass_##SUFFIX(int mode, bool xl, int n, const PassArgs<T> &a,           \
                                      int blocks, cudaStream_t s)                               \
     {                                                                                          \

@@ -3,4 +3,5 @@
 #include "pass_dispatch.cuh"
 namespace gpss {
 GPSS_DEFINE_PASS_DISPATCH(float, f32)
+GPSS_DEFINE_PIPE_DISPATCH(float, f32)
 }

@@ -32,9 +32,11 @@
 // Shared-memory layouts are chosen so every stage is bank-conflict free
 // (XL: one pad slot per N2-row plus N2 per line; COL: position-major).
 //
-// Constants (twiddles w_n^{r k1} and the kinetic phase factors) are held as
+// FP32 constants (twiddles w_n^{r k1} and the kinetic phase factors) are held as
 // double-word pairs hi + lo and applied with cmul2: a rounded constant alone
-// would repeat the same relative error on the same mode at every pass.
+// would repeat the same relative error on the same mode at every pass.  FP64
+// fields run the stages in 64-bit fixed point with 63-bit constants
+// (fft_fix.cuh); their field, epilogues and sums are FP64.
 //
 // Modes:
 //   MODE_FUSED  FFT -> phase -> iFFT (+ optional NL epilogue, reductions)
@@ -43,6 +45,7 @@
 //   MODE_DIAG   FFT only, writes nothing, accumulates Parseval sums (energy)
 #pragma once
 #include <cstdint>
+#include <type_traits>
 #include "fft_core.cuh"
 #include "fft_comp.cuh"
 #include "nl_phase.cuh"
@@ -242,12 +245,12 @@ template <typename V> struct __align__(2 * sizeof(V)) DWord {
 #ifndef GPSS_PASS_SM_THREADS_LEAN_XL_F32
 #define GPSS_PASS_SM_THREADS_LEAN_XL_F32 768  // 6 CTAs of 128
 #endif
-// FP64: CTAs of 64 threads.  The FP64 kernels are bound by GB300's FP64 rate
-// per SM, so small fields must spread over many SMs (2D 128^2 step 176 -> 88
-// us against 256-thread CTAs); 3D fields lose nothing (256^3 plain step 14.75
-// -> 14.38 ms, 128^3 fused 1015 -> 946 us).
+// FP64 fields (64-bit fixed point inside the pass): CTAs of 128 threads, so a
+// y/z access is a run of 8 adjacent cells (128 bytes).  The integer pipes, not
+// the field's traffic, bound these passes: three passes of a 256^3 step with
+// its FP64 nonlinear epilogue take 1.6 ms where FP64 transforms took 8 ms.
 #ifndef GPSS_PASS_THREADS_F64
-#define GPSS_PASS_THREADS_F64 64
+#define GPSS_PASS_THREADS_F64 128
 #endif
 // Small fields (a 2D y pass of 256 columns is 16 tiles of 16): y/z CTAs of 128
 // threads (FEAT_SMALL) give twice the tiles (2D 128^2 step 11.4 -> 10.6 us,
@@ -288,6 +291,11 @@ template <typename T, bool XL, int FEAT = 0> struct PassGeom {
 #ifndef GPSS_PASS_SM_THREADS_COMP_F32
 #define GPSS_PASS_SM_THREADS_COMP_F32 512
 #endif
+// FP64 passes hold every complex value as two 64-bit integers: 512 threads per
+// SM (128 registers, at most 100 bytes of spills in the largest instantiations).
+#ifndef GPSS_PASS_SM_THREADS_F64
+#define GPSS_PASS_SM_THREADS_F64 512
+#endif
 #ifndef GPSS_PASS_SM_THREADS_PLANE_XL_F32
 // stacked 2D planes: 7 CTAs per SM give 64 x 256^2 planes' 2048 x tiles 1.9
 // waves instead of 2.25 (the 512-run batch 44.1 -> 43.5 ms per 500 steps)
@@ -303,7 +311,8 @@ template <typename T, bool XL, int MODE, int FEAT> struct PassOcc {
         : (MODE == MODE_FUSED && XL && (FEAT & FEAT_PLANE))
             ? GPSS_PASS_SM_THREADS_PLANE_XL_F32
             : GPSS_PASS_SM_THREADS_F32;
-    static constexpr int MIN_BLOCKS = sizeof(T) == 4 ? SM_THREADS / PassGeom<T, XL, FEAT>::THREADS : 1;
+    static constexpr int MIN_BLOCKS =
+        (sizeof(T) == 4 ? SM_THREADS : GPSS_PASS_SM_THREADS_F64) / PassGeom<T, XL, FEAT>::THREADS;
 };
 
 template <int N> struct Split {
@@ -331,7 +340,9 @@ template <typename T, int N, bool XL, int FEAT = 0> struct PassShape {
     // w_n^{r k1} at k1*N2 + r (stage A) and at r*N1 + k1 (stage B) are the same
     // table when N1 == N2: then only one is held
     static constexpr bool TWB = N1 != N2;
-    static constexpr int SMEM_SLOTS = STAGE + DATA + (TWB ? 6 : 4) * N + (TMA ? 2 : 0);  // + tables hi and lo
+    // tables: hi and lo (FP32), or one 16-byte fixed-point constant (FP64)
+    static constexpr int TABLES = (TWB ? 3 : 2) * N * (sizeof(T) == 4 ? 2 : 1);
+    static constexpr int SMEM_SLOTS = STAGE + DATA + TABLES + (TMA ? 2 : 0);
     static constexpr size_t SMEM_BYTES = sizeof(vec2<T>) * SMEM_SLOTS;
 };
 
@@ -439,6 +450,7 @@ pass_kernel(const PassArgs<T> a)
     constexpr bool kMask = (FEAT & FEAT_MASK) != 0;
     constexpr bool kAcc = kDiag || (FEAT & FEAT_ACC) != 0;
     constexpr bool kComp = (FEAT & FEAT_COMP) != 0 && sizeof(T) == 4;
+    constexpr bool kFix = sizeof(T) == 8;  // FP64 fields: 64-bit fixed point inside the pass (fft_fix.cuh)
     static_assert(!kComp || (MODE == MODE_FUSED && !kMask && !kPlane && !kImagM), "compensated: fused kinetic passes");
     constexpr bool kTma = PassShape<T, N, XL, FEAT>::TMA;
     static_assert(!kTma || (MODE == MODE_FUSED && !kComp && !kDiag && !kPlane && !kImagM && !kMask && !kAdj),
@@ -446,6 +458,7 @@ pass_kernel(const PassArgs<T> a)
     const int red = a.red & ((kDiag ? (RED_POINT | RED_KIN) : 0) | (kNL || kDiag || kImagM ? RED_MASS : 0));
     const int64_t prow = kDiag ? a.prow : 0;
     using V = vec2<T>;
+    using E = typename std::conditional<kFix, int4, DWord<V>>::type;  // a table entry
     using S = PassShape<T, N, XL, FEAT>;
     constexpr int N1 = S::N1, N2 = S::N2, P = S::P, W = S::W, LS = S::LS;
     constexpr int THREADS = S::THREADS;
@@ -458,9 +471,11 @@ pass_kernel(const PassArgs<T> a)
     // layout of sdata with DATA1 such slots
     float4 *sd4 = reinterpret_cast<float4 *>(sdata);
     (void)sd4;
-    DWord<V> *stw = reinterpret_cast<DWord<V> *>(sdata + S::DATA);  // stage A [N], stage B [N]
-    DWord<V> *stwB = S::TWB ? stw + N : stw;
-    DWord<V> *sph = stw + (S::TWB ? 2 : 1) * N;                      // phase [N]
+    fxc *sfx = reinterpret_cast<fxc *>(sdata);  // FP64: the same slots hold fixed-point values
+    (void)sfx;
+    E *stw = reinterpret_cast<E *>(sdata + S::DATA);  // stage A [N], stage B [N]
+    E *stwB = S::TWB ? stw + N : stw;
+    E *sph = stw + (S::TWB ? 2 : 1) * N;                      // phase [N]
     uint64_t *tbar = reinterpret_cast<uint64_t *>(sph + N);           // FEAT_TMA copy barrier
     (void)tbar;
 
@@ -472,11 +487,23 @@ pass_kernel(const PassArgs<T> a)
         }
     }
     // tables into shared memory, hi/lo halves packed per entry
+    // (FP64: a fixed-point phase table starts with its power-of-two exponent)
+    const int4 *fxph = reinterpret_cast<const int4 *>(a.phase) + 1;
+    (void)fxph;
     for (int i = tid; i < N; i += THREADS) {
-        stw[i] = DWord<V>{a.tw[i], a.tw[N + i]};
-        if (S::TWB) stwB[i] = DWord<V>{a.tw[2 * N + i], a.tw[3 * N + i]};
-        if (MODE == MODE_FUSED && !kMask && prow == 0) sph[i] = DWord<V>{a.phase[i], a.phase[N + i]};
+        if constexpr (kFix) {
+            const int4 *ft = reinterpret_cast<const int4 *>(a.tw);
+            stw[i] = ft[i];
+            if (S::TWB) stwB[i] = ft[N + i];
+            if (MODE == MODE_FUSED && !kMask && prow == 0) sph[i] = fxph[i];
+        } else {
+            stw[i] = DWord<V>{a.tw[i], a.tw[N + i]};
+            if (S::TWB) stwB[i] = DWord<V>{a.tw[2 * N + i], a.tw[3 * N + i]};
+            if (MODE == MODE_FUSED && !kMask && prow == 0) sph[i] = DWord<V>{a.phase[i], a.phase[N + i]};
+        }
     }
+    const int fxpe = kFix && MODE == MODE_FUSED && !kMask ? reinterpret_cast<const int4 *>(a.phase)->x : 0;
+    (void)fxpe;
 
     const int w = XL ? tid / P : tid % W;
     const int r = XL ? tid % P : tid / W;
@@ -608,11 +635,188 @@ pass_kernel(const PassArgs<T> a)
                 }
             }
         }
-        if constexpr (!kComp) dft<N1, -1>(v);
+        if constexpr (!kComp && !kFix) dft<N1, -1>(v);
     }
     if constexpr (kTopBarrier) line_sync();  // the previous tile's stage B is done with sdata
 
-    if constexpr (kComp) {
+    if constexpr (kFix) {
+        // FP64 field: the same stages on 64-bit fixed-point values.  The tile's
+        // lines each take their quantum from their largest component.
+        constexpr int NI = N1 / N2;
+        if constexpr (MODE == MODE_INV) {
+#pragma unroll
+            for (int i = 0; i < NI; i++)
+#pragma unroll
+                for (int k2 = 0; k2 < N2; k2++)
+                    v[i * N2 + k2] = a.in[base + (uint32_t)((N2 == 1 ? 0 : r + P * i) + (N2 == 1 ? i : N1 * k2)) * st];
+        }
+        int word = fx_max_word<N1>(v);
+        if constexpr (XL) {
+#pragma unroll
+            for (int o = P / 2; o > 0; o >>= 1) word = max(word, __shfl_xor_sync(0xffffffffu, word, o));
+        } else {
+#pragma unroll
+            for (int o = 16; o >= W; o >>= 1) word = max(word, __shfl_xor_sync(0xffffffffu, word, o));
+        }
+        int ref = fx_ref(word);
+        float n2 = fx_norm2<N1>(v, ref);
+        if constexpr (XL) {
+#pragma unroll
+            for (int o = P / 2; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+        } else {
+#pragma unroll
+            for (int o = 16; o >= W; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+            if constexpr (P > 1) {
+                // columns: so far over the lanes of a warp that hold the same
+                // column, now across the CTA.  No further barrier is needed:
+                // every thread reads the sums before the barrier after stage
+                // A, and the next tile writes them after the one before stage
+                // C (or its top one)
+                __shared__ int sword[THREADS];
+                __shared__ float snorm[THREADS];
+                constexpr int G = W < 32 ? THREADS / 32 : P;
+                const int slot = W < 32 ? (tid >> 5) * W + w : tid;
+                if (W >= 32 || (tid & 31) < W) {
+                    sword[slot] = word;
+                    snorm[slot] = n2;
+                }
+                __syncthreads();
+                word = 0;
+#pragma unroll
+                for (int i = 0; i < G; i++) word = max(word, sword[i * W + w]);
+                ref = fx_ref(word);
+                n2 = 0.f;
+#pragma unroll
+                for (int i = 0; i < G; i++) {
+                    const int d = max(fx_ref(sword[i * W + w]) - ref, -50);
+                    n2 = fmaf(snorm[i * W + w], __int_as_float((127 + 2 * d) << 23), n2);
+                }
+            }
+        }
+        const bool bad = word >= 0x7ff00000;
+        const int q = fx_quantum(ref, n2);
+        fxc c[N1];
+#pragma unroll
+        for (int j = 0; j < N1; j++) {
+            c[j].x = fx_from(v[j].x, 1084 + q);
+            c[j].y = fx_from(v[j].y, 1084 + q);
+        }
+        // Parseval sums of the values X[k] of this thread (of quantum 2^qs)
+        auto kin = [&](const fxc &u, int k, const FxOut &os, T &s2, T &s1) {
+            const int kk = k < N / 2 ? k : k - N;
+            const T xi = (T)kk * kmult;
+            const V X = os(u);
+            const T m2 = X.x * X.x + X.y * X.y;
+            s2 += xi * xi * m2;
+            s1 += xi * m2;
+        };
+        auto kin_add = [&](T s2, T s1) {
+            acc_kin += s2 * (T)(1.0 / N);
+            if (a.coord) acc_rot += s1 * (T)(1.0 / N) * (T)a.coord[row];
+        };
+        (void)kin;
+        (void)kin_add;
+        int qo;  // the result's quantum
+        if constexpr (N2 == 1) {
+            // the whole line in this thread
+            if constexpr (MODE != MODE_INV) dft<N1, -1>(c);
+            if constexpr (MODE == MODE_FUSED || MODE == MODE_DIAG) {
+                if (red & RED_KIN) {
+                    const FxOut os(q, bad, 1.0, false);
+                    T s2 = 0, s1 = 0;
+#pragma unroll
+                    for (int k = 0; k < N1; k++) kin(c[k], k, os, s2, s1);
+                    kin_add(s2, s1);
+                }
+            }
+            if constexpr (MODE == MODE_FUSED) {
+                const int lim = kMask ? a.mask_lim[gg] : 0;
+#pragma unroll
+                for (int k = 0; k < N1; k++) {
+                    if constexpr (kMask) {
+                        c[k] = (k < (N + 1) / 2 ? k : N - k) <= lim ? fx_quarter(c[k]) : fxc{0, 0};
+                    } else {
+                        c[k] = fx_cmul<false>(c[k], prow ? fxph[row * prow + k] : sph[k]);
+                    }
+                }
+            }
+            if constexpr (MODE == MODE_FUSED || MODE == MODE_INV) dft<N1, +1>(c);
+            qo = q + (MODE == MODE_FUSED ? 2 + fxpe : 0);
+        } else {
+            // stage A: (k1, r) <- c[k1] w_n^{r k1} / 4
+            if constexpr (MODE != MODE_INV) {
+                dft<N1, -1>(c);
+#pragma unroll
+                for (int k1 = 0; k1 < N1; k1++) {
+                    const int m = k1 * N2 + r;
+                    sfx[sidx(m)] = k1 == 0 ? fx_quarter(c[0]) : fx_cmul<false>(c[k1], stw[m]);
+                }
+                line_sync();
+            }
+            // stage B: items k1 = r + P i
+            const FxOut os(q + 2, bad, 1.0, false);
+#pragma unroll
+            for (int i = 0; i < NI; i++) {
+                const int k1 = r + P * i;
+                fxc u[N2];
+                if constexpr (MODE == MODE_INV) {
+#pragma unroll
+                    for (int k2 = 0; k2 < N2; k2++) u[k2] = c[i * N2 + k2];
+                } else {
+#pragma unroll
+                    for (int rr = 0; rr < N2; rr++) u[rr] = sfx[sidx(k1 * N2 + rr)];
+                    dft<N2, -1>(u);  // u[k2] = X[k1 + N1 k2]
+                }
+                if constexpr (MODE == MODE_FWD) {
+                    if (valid) {
+#pragma unroll
+                        for (int k2 = 0; k2 < N2; k2++) a.out[base + (uint32_t)(k1 + N1 * k2) * st] = os(u[k2]);
+                    }
+                }
+                if constexpr (MODE == MODE_FUSED || MODE == MODE_DIAG) {
+                    if (red & RED_KIN) {
+                        T s2 = 0, s1 = 0;
+#pragma unroll
+                        for (int k2 = 0; k2 < N2; k2++) kin(u[k2], k1 + N1 * k2, os, s2, s1);
+                        kin_add(s2, s1);
+                    }
+                }
+                if constexpr (MODE == MODE_FUSED) {
+                    const int lim = kMask ? a.mask_lim[gg] : 0;
+#pragma unroll
+                    for (int k2 = 0; k2 < N2; k2++) {
+                        const int k = k1 + N1 * k2;
+                        if constexpr (kMask) {
+                            u[k2] = (k < (N + 1) / 2 ? k : N - k) <= lim ? fx_quarter(u[k2]) : fxc{0, 0};
+                        } else {
+                            u[k2] = fx_cmul<false>(u[k2], prow ? fxph[row * prow + k] : sph[k]);
+                        }
+                    }
+                }
+                if constexpr (MODE == MODE_FUSED || MODE == MODE_INV) {
+                    dft<N2, +1>(u);  // u[rr] = Z[k1][rr]
+#pragma unroll
+                    for (int rr = 0; rr < N2; rr++)
+                        sfx[sidx(k1 * N2 + rr)] = rr == 0 ? fx_quarter(u[0]) : fx_cmul<true>(u[rr], stwB[rr * N1 + k1]);
+                }
+            }
+            if constexpr (MODE == MODE_FUSED || MODE == MODE_INV) {
+                line_sync();
+                // stage C
+#pragma unroll
+                for (int k1 = 0; k1 < N1; k1++) c[k1] = sfx[sidx(k1 * N2 + r)];
+                dft<N1, +1>(c);
+            }
+            qo = q + (MODE == MODE_FUSED ? 6 + fxpe : 2);
+        }
+        if constexpr (MODE != MODE_DIAG && !(MODE == MODE_FWD && N2 > 1)) {
+            // 1/n of the inverse, and the deferred factor
+            const FxOut oc(MODE == MODE_FWD ? qo : qo - FxLog<N>::V, bad, (double)tscale,
+                           MODE == MODE_FUSED && tscaled);
+#pragma unroll
+            for (int j = 0; j < N1; j++) v[j] = oc(c[j]);
+        }
+    } else if constexpr (kComp) {
         // compensated kinetic pass: the same stages on gridded two-float
         // values (fft_comp.cuh); each thread grids each stage's values on its
         // own quantum.  The deferred factor enters with the first gridding

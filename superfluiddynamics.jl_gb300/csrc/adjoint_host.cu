@@ -51,12 +51,8 @@ static int adj_group(gpss_ctx *c, void *buf, double dtl, bool reverse, bool nl, 
         // stay bitwise those of the forward)
         a.comp = sizeof(T) == 4 && (c->flags & GPSS_FLAG_COMPENSATED) != 0;
         if (step == c->ndim - 1 && (nl || adj_pre)) {
-            a.V = c->have_V ? (const T *)c->V : nullptr;
-            a.nl_beta = c->beta;
-            a.nl_dt = dtnl;
-            a.nl_split = nl_split(c->beta, dtnl);
+            GPSS_TRY(set_nl<T>(c, axis, a, nl ? NL_REAL : NL_NONE, dtnl));
             if (nl) {
-                a.nl_mode = NL_REAL;
                 a.pre_out = (vec2<T> *)pre_out;
             } else {
                 a.adj_pre = (const vec2<T> *)adj_pre;

@@ -75,6 +75,16 @@ struct gpss_ctx {
     int *status = nullptr;    // [1]
     unsigned int *counter = nullptr;  // arrival counter of the in-kernel reduction finish
     std::vector<PhaseEntry> phases;
+    // FP64 fields: what the fixed-point nonlinear flow reads besides the field
+    // -- roots of unity, and per time step V dt in turns (set_nl); vbad: V
+    // holds NaN or infinity
+    struct VturnEntry {
+        double dt;
+        void *dev;
+    };
+    std::vector<VturnEntry> vturns;
+    void *nl_tab = nullptr;
+    int *vbad = nullptr;
     void *rk_buf[4] = {nullptr, nullptr, nullptr, nullptr};  // RK: stage state, lapRot, NL term, sum
     int *rk_lim = nullptr;    // RK: 2/3-rule limits per inner position (the FEAT_MASK pass)
     void *im_buf = nullptr;   // implicit schemes: work fields (implicit_impl)
@@ -319,6 +329,85 @@ static std::string graph_key(const char *what, std::initializer_list<double> v)
 static const int64_t kGraphCells = int64_t(1) << 21;
 static const int kGraphChunk = 32;  // time steps per captured chunk
 
+// The table V dt / (2 pi) of a time step (fft_fix.cuh), made on its first use
+// after the potential was set.  Graphs hold its address, so the tables of up
+// to four time steps are kept (a program that alternates between two finds
+// both); a fifth takes the place of the oldest, and the graphs go.
+static int get_vturn(gpss_ctx *c, double dt, const long long **dev)
+{
+    for (auto &e : c->vturns)
+        if (e.dt == dt) {
+            *dev = (const long long *)e.dev;
+            return GPSS_OK;
+        }
+    void *buf = nullptr;
+    if (c->vturns.size() >= 4) {
+        clear_graphs(c);  // the stream orders the overwrite behind earlier launches
+        buf = c->vturns.front().dev;
+        c->vturns.erase(c->vturns.begin());
+    } else {
+        GPSS_TRY(dev_alloc(c, &buf, (size_t)c->total * sizeof(long long)));
+    }
+    c->vturns.push_back({dt, buf});
+    int64_t m;
+    int e;
+    fx_turns((ldouble)dt, m, e);
+    CUDA_TRY(c, launch_vturn((const double *)c->V, (long long *)buf, m, e, c->total, c->vbad, c->stream));
+    c->launches++;
+    *dev = (const long long *)buf;
+    return GPSS_OK;
+}
+
+// forget the tables of the previous potential (their buffers are freed)
+static void clear_vturns(gpss_ctx *c)
+{
+    if (c->vturns.empty()) return;
+    clear_graphs(c);
+    if (c->stream) cudaStreamSynchronize(c->stream);
+    for (auto &e : c->vturns) {
+        cudaFree(e.dev);
+        c->bytes -= (int64_t)((size_t)c->total * sizeof(long long));
+    }
+    c->vturns.clear();
+}
+
+// the nonlinear flow N(dt) as the epilogue of a pass
+template <typename T> static int set_nl(gpss_ctx *c, int axis, PassArgs<T> &a, int mode, double dt)
+{
+    a.nl_mode = mode;
+    a.V = c->have_V ? (const T *)c->V : nullptr;
+    a.nl_beta = c->beta;
+    a.nl_dt = dt;
+    a.nl_split = nl_split(c->beta, dt);
+    if (!fx_axis(c, axis) || mode != NL_REAL) return GPSS_OK;
+    // FP64 register pass: the flow in fixed point
+    if (!c->nl_tab) {
+        std::vector<int4> t(FX_NL_TAB);
+        for (int k = 0; k < FX_NL_TAB; k++) {
+            ldouble cs, sn;
+            unit_root(k, FX_NL_TAB, &cs, &sn);
+            t[(size_t)k] = fx_const(cs, sn);
+        }
+        GPSS_TRY(upload_fx(c, &c->nl_tab, t));
+    }
+    int64_t m;
+    int e;
+    fx_turns((ldouble)c->beta * (ldouble)dt, m, e);
+    a.nl_fx.gl = (int)(uint32_t)m;
+    a.nl_fx.gh = (int)((m - (int64_t)a.nl_fx.gl) >> 32);
+    a.nl_fx.ge = e;
+    a.nl_fx.tab = (const int4 *)c->nl_tab;
+    if (c->have_V) {
+        if (!c->vbad) {
+            GPSS_TRY(dev_alloc(c, (void **)&c->vbad, sizeof(int)));
+            CUDA_TRY(c, cudaMemsetAsync(c->vbad, 0, sizeof(int), c->stream));
+        }
+        GPSS_TRY(get_vturn(c, dt, &a.nl_fx.vturn));
+        a.nl_fx.vbad = c->vbad;
+    }
+    return GPSS_OK;
+}
+
 template <typename T> static PassArgs<T> axis_args(gpss_ctx *c, int axis, const void *in, void *out)
 {
     PassArgs<T> a;
@@ -462,13 +551,7 @@ static int kinetic_fused(gpss_ctx *c, double dtl, int imag, bool nl, double dtnl
         }
         if (prescale && step == 0) a.scale = c->scale;
         const bool last = step == c->ndim - 1;
-        if (last && nl) {
-            a.nl_mode = imag ? NL_IMAG : NL_REAL;
-            a.V = c->have_V ? (const T *)c->V : nullptr;
-            a.nl_beta = c->beta;
-            a.nl_dt = dtnl;
-            a.nl_split = nl_split(c->beta, dtnl);
-        }
+        if (last && nl) GPSS_TRY(set_nl<T>(c, axis, a, imag ? NL_IMAG : NL_REAL, dtnl));
         if (last) a.red |= red_last;
         if (a.red & RED_POINT) a.V = c->have_V ? (const T *)c->V : nullptr;
         if (diag_kin) {

@@ -99,12 +99,7 @@ static int imag_flow(gpss_ctx *c, double dtl, const void *in0, bool pre_nl, void
         const void *ph;
         GPSS_TRY(get_phase(c, axis, dtl, 1, 1, &ph, &a.prow));
         a.phase = (const vec2<T> *)ph;
-        if ((first && pre_nl) || (last && nl_last)) {
-            a.V = c->have_V ? (const T *)c->V : nullptr;
-            a.nl_beta = c->beta;
-            a.nl_dt = dtnl;
-            a.nl_split = nl_split(c->beta, dtnl);
-        }
+        if ((first && pre_nl) || (last && nl_last)) GPSS_TRY(set_nl<T>(c, axis, a, NL_NONE, dtnl));
         if (first && pre_nl) {
             a.nl_pre = 1;
             a.scale = c->scale;
@@ -384,10 +379,11 @@ void gpss_destroy(gpss_ctx *c)
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     clear_phases(c);  // and the graphs
+    clear_vturns(c);
     void *ptrs[] = {c->psi, c->scratch, c->V, c->tw[0], c->tw[1], c->tw[2], c->coord_dev[0],
                     c->coord_dev[1], c->coord_dev[2], c->partials, c->sums, c->scale, c->status,
                     c->counter, c->rk_buf[0], c->rk_buf[1], c->rk_buf[2], c->rk_buf[3], c->rk_lim,
-                    c->adj_buf, c->im_buf, c->tmap_dev};
+                    c->adj_buf, c->im_buf, c->tmap_dev, c->nl_tab, c->vbad};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     for (auto &e : c->ev)
@@ -542,6 +538,8 @@ int gpss_set_potential(gpss_ctx *c, const double *V)
     CUDA_TRY(c, cudaSetDevice(c->device));
     GPSS_TRY(flush_pending(c));
     clear_graphs(c);
+    clear_vturns(c);
+    if (c->vbad) CUDA_TRY(c, cudaMemsetAsync(c->vbad, 0, sizeof(int), c->stream));
     if (!V) { c->have_V = false; return GPSS_OK; }
     if (!c->V) GPSS_TRY(dev_alloc(c, &c->V, (size_t)c->total * real_bytes(c)));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
@@ -803,13 +801,7 @@ int gpss_time_pass(gpss_ctx *c, int axis, int mode, int reps, double dt, double 
             a.fin_status = c->status;
             CUDA_TRY(c, cudaMemsetAsync(c->status, 0, sizeof(int), c->stream));
         }
-        if (mode == 1) {
-            a.nl_mode = NL_REAL;
-            a.V = c->have_V ? (const T *)c->V : nullptr;
-            a.nl_beta = c->beta;
-            a.nl_dt = dt;
-            a.nl_split = nl_split(c->beta, dt);
-        }
+        if (mode == 1) GPSS_TRY(set_nl<T>(c, axis, a, NL_REAL, dt));
         GPSS_TRY(launch<T>(c, axis, MODE_FUSED, a));  // warm-up
         CUDA_TRY(c, cudaEventRecord(c->ev[6], c->stream));
         for (int i = 0; i < reps; i++) GPSS_TRY(launch<T>(c, axis, MODE_FUSED, a));

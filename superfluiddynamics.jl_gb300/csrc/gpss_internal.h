@@ -127,6 +127,18 @@ inline std::vector<int4> fx_phase_table(const std::vector<long double> &re, cons
     return t;
 }
 
+// x / (2 pi) as m 2^e with m of 62 bits and a sign (0: m = 0)
+inline void fx_turns(long double x, int64_t &m, int &e)
+{
+    const long double two_pi = 6.283185307179586476925286766559005768L;
+    m = 0;
+    e = 0;
+    if (x == 0.0L) return;
+    const long double f = frexpl(x / two_pi, &e);
+    m = (int64_t)llroundl(ldexpl(f, 62));
+    e -= 62;
+}
+
 // pass launchers (pass_f32.cu / pass_f64.cu)
 cudaError_t launch_pass_f32(int mode, bool xl, int n, const PassArgs<float> &a, int blocks,
                             cudaStream_t s);
@@ -185,6 +197,8 @@ inline bool reg_line(int64_t n) { return n >= 2 && n <= 256 && (n & (n - 1)) == 
 // pointwise kernels (pointwise.cu)
 cudaError_t launch_f64_to_f32(const double *in, float *out, int64_t count, cudaStream_t s);
 cudaError_t launch_f32_to_f64(const float *in, double *out, int64_t count, cudaStream_t s);
+cudaError_t launch_vturn(const double *V, long long *out, long long d, int de, int64_t count, int *bad,
+                         cudaStream_t s);
 template <typename T>
 cudaError_t launch_mul_phase(vec2<T> *data, const vec2<T> *phase, int64_t prow, int axis,
                              const int64_t *n, int64_t total, cudaStream_t s);

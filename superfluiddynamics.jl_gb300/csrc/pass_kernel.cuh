@@ -149,6 +149,7 @@ template <typename T> struct PassArgs {
     const T *V;              // nullable (zero potential)
     double nl_beta, nl_dt;
     NLSplit nl_split;        // FP32 kernels: beta, dt, beta*dt as float pairs
+    FxNlArgs nl_fx;          // FP64 register passes, real time: the flow in fixed point
     // deferred renormalisation: multiply the input by the factor in a
     // ScaleCell (nullable; `scale` points at its FP64 member)
     const double *scale;
@@ -341,7 +342,9 @@ template <typename T, int N, bool XL, int FEAT = 0> struct PassShape {
     // table when N1 == N2: then only one is held
     static constexpr bool TWB = N1 != N2;
     // tables: hi and lo (FP32), or one 16-byte fixed-point constant (FP64)
-    static constexpr int TABLES = (TWB ? 3 : 2) * N * (sizeof(T) == 4 ? 2 : 1);
+    // and, where the pass may carry the nonlinear flow, its roots of unity
+    static constexpr int NLTAB = sizeof(T) == 8 && (FEAT & FEAT_NL) != 0 ? FX_NL_TAB : 0;
+    static constexpr int TABLES = (TWB ? 3 : 2) * N * (sizeof(T) == 4 ? 2 : 1) + NLTAB;
     static constexpr int SMEM_SLOTS = STAGE + DATA + TABLES + (TMA ? 2 : 0);
     static constexpr size_t SMEM_BYTES = sizeof(vec2<T>) * SMEM_SLOTS;
 };
@@ -502,6 +505,14 @@ pass_kernel(const PassArgs<T> a)
             if (MODE == MODE_FUSED && !kMask && prow == 0) sph[i] = DWord<V>{a.phase[i], a.phase[N + i]};
         }
     }
+    // the nonlinear flow in fixed point (FP64, real time)
+    const bool fxnl = kFix && kNL && MODE == MODE_FUSED && a.nl_mode == NL_REAL;
+    int4 *snl = reinterpret_cast<int4 *>(sph + N);
+    (void)snl;
+    if constexpr (kFix && kNL && MODE == MODE_FUSED) {
+        if (fxnl)
+            for (int i = tid; i < FX_NL_TAB; i += THREADS) snl[i] = a.nl_fx.tab[i];
+    }
     const int fxpe = kFix && MODE == MODE_FUSED && !kMask ? reinterpret_cast<const int4 *>(a.phase)->x : 0;
     (void)fxpe;
 
@@ -521,6 +532,8 @@ pass_kernel(const PassArgs<T> a)
     const bool scaled = a.scale != nullptr;
     const T scale = scaled ? load_scale<T>(a.scale) : (T)1;
     const T kmult = a.kmult;
+    const bool vbad = fxnl && a.nl_fx.vbad && *a.nl_fx.vbad != 0;
+    (void)vbad;
     // compensated passes with a mass bound: one grid for every stage (C of
     // the quantum 2^-22 of 32 sqrt(M/2) = 16 sqrt(2 M), rounded up)
     constexpr bool gridm = kComp && (FEAT & FEAT_GRIDM) != 0;
@@ -811,8 +824,34 @@ pass_kernel(const PassArgs<T> a)
         }
         if constexpr (MODE != MODE_DIAG && !(MODE == MODE_FWD && N2 > 1)) {
             // 1/n of the inverse, and the deferred factor
-            const FxOut oc(MODE == MODE_FWD ? qo : qo - FxLog<N>::V, bad, (double)tscale,
-                           MODE == MODE_FUSED && tscaled);
+            int qv = MODE == MODE_FWD ? qo : qo - FxLog<N>::V;
+            if constexpr (MODE == MODE_FUSED && kNL) {
+                if (fxnl) {
+                    if constexpr (kAdj) {
+                        if (a.pre_out && valid) {
+                            const FxOut op(qv, bad, 1.0, false);
+#pragma unroll
+                            for (int j = 0; j < N1; j++) a.pre_out[base + (uint32_t)(r + N2 * j) * st] = op(c[j]);
+                        }
+                    }
+                    // the values are below 2^60 n / 64 (whole line in a
+                    // thread: n / 4): shorter lines have room for more bits
+                    constexpr int KS = 2 - (FxLog<N>::V - (N2 > 1 ? 6 : 2));
+                    qv -= KS;
+                    const int sh = 190 + 2 * qv + a.nl_fx.ge;
+                    const int lsh = min(max(sh, 0), 63), rsh = min(max(-sh, 0), 63);
+#pragma unroll
+                    for (int j = 0; j < N1; j++) {
+                        const long long vt =
+                            a.nl_fx.vturn ? a.nl_fx.vturn[base + (uint32_t)(r + N2 * j) * st] : 0;
+                        c[j].x <<= KS;
+                        c[j].y <<= KS;
+                        c[j] = fx_nl_real(c[j], vt, a.nl_fx.gh, a.nl_fx.gl, lsh, rsh, snl);
+                    }
+                    qv += 2;
+                }
+            }
+            const FxOut oc(qv, bad || vbad, (double)tscale, MODE == MODE_FUSED && tscaled);
 #pragma unroll
             for (int j = 0; j < N1; j++) v[j] = oc(c[j]);
         }
@@ -1110,7 +1149,7 @@ pass_kernel(const PassArgs<T> a)
     // ---- epilogue: positions r + N2 j
     if constexpr (MODE == MODE_FUSED || MODE == MODE_INV) {
         if constexpr (MODE == MODE_FUSED && kAdj) {
-            if (a.pre_out && valid) {
+            if (a.pre_out && valid && !fxnl) {  // (fixed point: stored above)
 #pragma unroll
                 for (int j = 0; j < N1; j++) a.pre_out[base + (uint32_t)(r + N2 * j) * st] = v[j];
             }
@@ -1132,7 +1171,7 @@ pass_kernel(const PassArgs<T> a)
             }
         }
         if constexpr (MODE == MODE_FUSED) {
-            if (kNL && a.nl_mode != NL_NONE) {
+            if (kNL && a.nl_mode != NL_NONE && !fxnl) {
                 const NLConst<T> nlc =
                     nl_const<T>(kPlane ? a.plane_nl[plane] : a.nl_split, a.nl_beta, a.nl_dt);
                 const bool imag = a.nl_mode == NL_IMAG;

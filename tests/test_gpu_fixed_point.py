@@ -77,3 +77,54 @@ def test_zero_lines_stay_zero(sfd):
     psi = np.zeros(shape, dtype=np.complex128)
     got = run_model(sfd, shape, BOUNDS, psi, coeffD=CD, beta=0.0, dt=DT, nsteps=1, precision="fp64")
     assert (got == 0).all()
+
+
+@pytest.mark.parametrize("beta,vmax,dt", [(0.0, 3.0, 1e-3), (20.0, 0.0, 1e-3), (-20.0, 3.0, 0.4), (500.0, 1e4, 0.7),
+                                          (1e-9, 1e-9, 1e-3), (20.0, 3.0, -0.05)])
+@pytest.mark.parametrize("shape", [(4, 2), (16, 16), (8, 32), (32, 64), (16, 128), (64, 256)])
+def test_nonlinear_flow(sfd, shape, beta, vmax, dt):
+    """exp(-i (V + beta |psi|^2) dt) psi alone (coeffD = 0: the kinetic flows
+    are the identity) against long double."""
+    rng = np.random.default_rng(7 * sum(shape))
+    psi = field("random", shape, rng)
+    V = np.asfortranarray(rng.uniform(-vmax, vmax, shape)) if vmax else None
+    got = run_model(sfd, shape, BOUNDS, psi, coeffD=0.0, beta=beta, V=V, dt=dt, nsteps=1, precision="fp64")
+    q = psi.astype(np.clongdouble)
+    rho = q.real ** 2 + q.imag ** 2
+    b, d = np.longdouble(beta), np.longdouble(dt)
+    exact = q * np.exp(np.clongdouble(-1j) * ((0 if V is None else V.astype(np.longdouble)) + b * rho) * d)
+    # The passes as above.  theta: two of them come before the flow, so psi
+    # enters |psi|^2 with 2 x 1.27e-16 of relative error at most and theta with
+    # twice that; |psi|^2 itself carries 62 bits below the line's largest
+    # possible value n rms^2 <= 2^8 rms^2, 4 units of 2^-54 rms^2 for its
+    # rounding, its low product and the factor's (the potential's part is exact).
+    w = np.abs(psi) / np.linalg.norm(psi)
+    theta = abs(beta * dt) * float(np.linalg.norm(w * rho.astype(np.float64)))
+    assert rel(got, exact) < 5.1e-16 + 5.1e-16 * theta + 4 * 2.0 ** -54 * abs(beta * dt) * float(rho.mean())
+
+
+def test_nonlinear_flow_with_a_nonfinite_potential(sfd):
+    shape = (32, 16)
+    V = np.zeros(shape, order="F")
+    V[3, 4] = np.nan
+    got = run_model(sfd, shape, BOUNDS, field("random", shape, np.random.default_rng(2)), V=V, nsteps=1)
+    assert not np.isfinite(got).any()
+
+
+def test_time_steps_in_turn(sfd):
+    """A model whose calls alternate between more time steps than it keeps
+    potential tables for gives what models of one time step each give."""
+    shape, rng = (32, 64), np.random.default_rng(5)
+    psi, V = field("random", shape, rng), np.asfortranarray(rng.uniform(0.0, 50.0, shape))
+    g = sfd.Grid(shape, BOUNDS)
+    f = sfd.Field(g)
+    f.phi = psi
+    n = sfd.NumModelSplit2(f, sfd.GrossPitaevskiiParameters(sfd.PotentialArray(f, V), coeffD=CD, beta=2.0), 1e-3, 1, 1)
+    want = psi
+    for dt in [1e-3, 2e-3, 1e-3, 3e-3, 4e-3, 5e-3, 1e-3, 2e-3, 1e-3]:
+        n.dt = dt
+        n.step(70)
+        got = f.phi.copy(order="F")
+        want = run_model(sfd, shape, BOUNDS, want, coeffD=CD, beta=2.0, V=V, dt=dt, nsteps=70)
+        assert np.array_equal(got, want)
+    n.close()

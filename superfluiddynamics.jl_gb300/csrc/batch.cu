@@ -475,7 +475,7 @@ static int build_tables(gpss_batch *b, double dt)
     for (size_t si = 0; si < b->set_keys.size(); si++) {
         const int64_t n = b->set_keys[si].first;
         std::vector<ldouble> re, im;
-        twiddle_rows(n, re, im);
+        twiddle_rows(n, 4, re, im);
         int rc = upload(b, dw_table(re, im, n), &sets[si].tw);
         if (rc) return rc;
         for (int axis = 0; axis < 2; axis++) {

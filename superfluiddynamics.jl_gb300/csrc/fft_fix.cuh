@@ -71,15 +71,13 @@ __device__ __forceinline__ long long fx_rmul(long long a, int rh, int rl)
 
 // A table constant: 2^62 times a complex number of modulus at most 1, the
 // halves of each component signed (c = h 2^32 + l).
-// a * c / 4 and a * conj(c) / 4
-template <bool CONJ> __device__ __forceinline__ fxc fx_cmul(fxc a, int4 c)
+// a * c / 4
+__device__ __forceinline__ fxc fx_cmul(fxc a, int4 c)
 {
     int xh, xl, yh, yl;
     fx_split(a.x, xh, xl);
     fx_split(a.y, yh, yl);
-    const int rl = c.x, rh = c.y;
-    const int pl = CONJ ? -c.z : c.z, ph = CONJ ? -c.w : c.w;    // imaginary part
-    const int ml = CONJ ? c.z : -c.z, mh = CONJ ? c.w : -c.w;    // minus it
+    const int rl = c.x, rh = c.y, pl = c.z, ph = c.w, ml = -c.z, mh = -c.w;
     fxc o;
     o.x = fx_fold(fx_madw(xh, rh, fx_madw(yh, mh, FX_S0)),
                   fx_madw(xl, rh, fx_madw(yl, mh, fx_madw(xh, rl, fx_madw(yh, ml, FX_X0)))));
@@ -266,7 +264,7 @@ __device__ __forceinline__ fxc fx_nl_real(fxc c, long long vt, int gh, int gl, i
     fx_split(s1, ch, cl);
     const long long si = fx_rmul(u, ch, cl);
     // exp(i theta) in units of 2^-62
-    fxc f = fx_cmul<false>(fxc{co, si}, tab[k & (FX_NL_TAB - 1)]);
+    fxc f = fx_cmul(fxc{co, si}, tab[k & (FX_NL_TAB - 1)]);
     f.x <<= 2;
     f.y <<= 2;
     // c conj(f) / 4 (run-time constants are negated whole, not by halves: a
@@ -283,33 +281,54 @@ __device__ __forceinline__ fxc fx_nl_real(fxc c, long long vt, int gh, int gl, i
     return o;
 }
 
-// Leaving fixed point: an integer v times 2^q as the FP64 nearest to it.  The
-// halves of v are placed in the significands of 2^84 2^q and 2^52 2^q, so two
-// additions (the first exact) give the value; q outside the range that their
-// exponents leave is applied as a second factor.
+// Leaving fixed point: an integer v times 2^q as the FP64 nearest to it, in two
+// ways.  fp: the halves of v are placed in the significands of 2^84 2^q and 2^52
+// 2^q, so two FP64 additions (the first exact) give the value.  integer: the
+// magnitude, normalised by its leading zeros and rounded at bit 11, under the
+// exponent.  Additions alone keep the narrow FP64 pipe busy for half of a 256^3
+// pass and are the longest part of one warp's work on a small field; integers
+// alone are some 40 instructions per cell.  All additions / half / a quarter /
+// none, us per pass: 256^3 x 306 / 292 / 306 / 325, 128^3 43.5 / 38.6 / 39.1 /
+// 40.0, 64^3 8.4 / 7.2 / 6.8 / 6.7: half of them for lines of 256, else a quarter.
+// q outside the range that the exponents leave is applied as a second factor.
 struct FxOut {
-    int hw, lw;
+    int qc;
     double k, f;
-    bool scaled;
-    __device__ __forceinline__ FxOut(int q, bool bad, double scale, bool with_scale)
+    bool scaled, bad;
+    __device__ __forceinline__ FxOut(int q, bool bad_, double scale, bool with_scale) : bad(bad_)
     {
-        const int qc = min(max(q, -1000), 900), d = min(max(q - qc, -1000), 1000);
-        hw = 0x45300000 + qc * (1 << 20);
-        lw = 0x43300000 + qc * (1 << 20);
-        k = bad ? __longlong_as_double(0x7ff8000000000000LL)
-                : __hiloint2double(0x45300000 + qc * (1 << 20), (int)0x80100000);
+        qc = min(max(q, -900), 900);
+        const int d = min(max(q - qc, -1000), 1000);
+        k = __hiloint2double(0x45300000 + qc * (1 << 20), (int)0x80100000);
         scaled = with_scale || d != 0;
         f = __hiloint2double((1023 + d) << 20, 0) * scale;
     }
-    __device__ __forceinline__ double real(long long v) const
+    __device__ __forceinline__ double fp(long long v) const
     {
-        const double h = __hiloint2double(hw, (int)((unsigned)(v >> 32) ^ 0x80000000u));
-        const double l = __hiloint2double(lw, (int)v);
+        const double h = __hiloint2double(0x45300000 + qc * (1 << 20), (int)((unsigned)(v >> 32) ^ 0x80000000u));
+        const double l = __hiloint2double(0x43300000 + qc * (1 << 20), (int)v);
         return (h - k) + l;
     }
-    __device__ __forceinline__ double2 operator()(fxc c) const
+    __device__ __forceinline__ double integer(long long v) const
     {
-        double2 o = make_double2(real(c.x), real(c.y));
+        const int sg = (int)(v >> 63);
+        const unsigned long long m = (unsigned long long)((v ^ (long long)sg) - (long long)sg);
+        const unsigned mh = (unsigned)(m >> 32), ml = (unsigned)m;
+        const bool small = mh == 0;
+        const int z = __clz((int)(small ? ml : mh));
+        const unsigned nh = small ? ml << (z & 31) : __funnelshift_l(ml, mh, z);
+        const unsigned nl = small ? 0u : ml << z;
+        // the top bit, at 63, becomes the significand's implicit one
+        const unsigned lo = __funnelshift_r(nl, nh, 11), r = lo + ((nl >> 10) & 1u);
+        const unsigned e = (unsigned)((1023 + 62 + qc - z - (small ? 32 : 0)) << 20) | ((unsigned)sg & 0x80000000u);
+        const unsigned hi = (nh >> 11) + e + (r < lo ? 1u : 0u);
+        return m == 0 ? 0.0 : __hiloint2double((int)hi, (int)r);
+    }
+    // with_fp: the real part by additions
+    __device__ __forceinline__ double2 operator()(fxc c, bool with_fp) const
+    {
+        double2 o = make_double2(with_fp ? fp(c.x) : integer(c.x), integer(c.y));
+        if (bad) o.x = o.y = __longlong_as_double(0x7ff8000000000000LL);
         if (scaled) {
             o.x *= f;
             o.y *= f;

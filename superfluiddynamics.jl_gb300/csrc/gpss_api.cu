@@ -479,7 +479,7 @@ int gpss_create(gpss_ctx **out, int ndim, const int64_t *n, const double *lo, co
             if ((rc = upload_dw(c, &c->tw[a], re, im, 1, na))) return bail(rc);
         } else {
             // two rows: stage-A order (k1*N2 + r) and stage-B order (r*N1 + k1)
-            twiddle_rows(na, re, im);
+            twiddle_rows(na, precision == GPSS_FP64 ? 8 : 4, re, im);
             if ((rc = fx_axis(c, a) ? upload_fx(c, &c->tw[a], fx_table(re, im))
                                     : upload_dw(c, &c->tw[a], re, im, 2, na)))
                 return bail(rc);

@@ -38,10 +38,10 @@ inline void unit_root(int64_t k, int64_t n, long double *cs, long double *sn)
 
 // The twiddles w_n^{r k1} = exp(-2 pi i r k1 / n) of a line of n cells in the
 // pass kernel's two orders: row 0 at m = k1*N2 + r (stage A), row 1 at
-// m = r*N1 + k1 (stage B), N1 = min(n, 16), N2 = n / N1.
-inline void twiddle_rows(int64_t n, std::vector<long double> &re, std::vector<long double> &im)
+// m = r*N1 + k1 (stage B), N1 of the passes of a precision (split_n1), N2 = n / N1.
+inline void twiddle_rows(int64_t n, int precision_bytes, std::vector<long double> &re, std::vector<long double> &im)
 {
-    const int64_t N1 = n <= 16 ? n : 16, N2 = n / N1;
+    const int64_t N1 = split_n1(n, precision_bytes), N2 = n / N1;
     re.assign((size_t)(2 * n), 0.0L);
     im.assign((size_t)(2 * n), 0.0L);
     for (int64_t k1 = 0; k1 < N1; k1++)

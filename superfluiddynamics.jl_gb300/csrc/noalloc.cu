@@ -83,7 +83,7 @@ int noalloc_fail(int code, const char *msg, cudaError_t e = cudaSuccess)
 template <typename T> std::vector<unsigned char> twiddle_table(int64_t n)
 {
     std::vector<long double> re, im;
-    twiddle_rows(n, re, im);
+    twiddle_rows(n, (int)sizeof(T), re, im);
     auto bytes = [](const auto &t) {
         const unsigned char *p = reinterpret_cast<const unsigned char *>(t.data());
         return std::vector<unsigned char>(p, p + t.size() * sizeof(t[0]));

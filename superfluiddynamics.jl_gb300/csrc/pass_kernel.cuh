@@ -316,14 +316,18 @@ template <typename T, bool XL, int MODE, int FEAT> struct PassOcc {
         (sizeof(T) == 4 ? SM_THREADS : GPSS_PASS_SM_THREADS_F64) / PassGeom<T, XL, FEAT>::THREADS;
 };
 
-template <int N> struct Split {
-    static constexpr int N1 = N <= 16 ? N : 16;
+// (FP64 lines of 32 and 64 cells split 8 x 4 and 8 x 8: twice the threads per
+// line and half the registers, 64^2 10.3 -> 5.8 us per pass, 64^3 11.1 -> 8.4;
+// the host's tables follow split_n1)
+constexpr int split_n1(int64_t n, int bytes) { return n <= 16 ? (int)n : (bytes == 8 && n <= 64) ? 8 : 16; }
+template <int N, int BYTES = 4> struct Split {
+    static constexpr int N1 = split_n1(N, BYTES);
     static constexpr int N2 = N / N1;
 };
 
 template <typename T, int N, bool XL, int FEAT = 0> struct PassShape {
-    static constexpr int N1 = Split<N>::N1;
-    static constexpr int N2 = Split<N>::N2;
+    static constexpr int N1 = Split<N, sizeof(T)>::N1;
+    static constexpr int N2 = Split<N, sizeof(T)>::N2;
     static constexpr int P = N2;                       // threads per line
     static constexpr int THREADS = PassGeom<T, XL, FEAT>::THREADS;
     static constexpr int W = THREADS / P;              // lines per CTA
@@ -718,7 +722,7 @@ pass_kernel(const PassArgs<T> a)
         auto kin = [&](const fxc &u, int k, const FxOut &os, T &s2, T &s1) {
             const int kk = k < N / 2 ? k : k - N;
             const T xi = (T)kk * kmult;
-            const V X = os(u);
+            const V X = os(u, false);
             const T m2 = X.x * X.x + X.y * X.y;
             s2 += xi * xi * m2;
             s1 += xi * m2;
@@ -729,109 +733,188 @@ pass_kernel(const PassArgs<T> a)
         };
         (void)kin;
         (void)kin_add;
-        int qo;  // the result's quantum
-        if constexpr (N2 == 1) {
-            // the whole line in this thread
-            if constexpr (MODE != MODE_INV) dft<N1, -1>(c);
+        // One transform routine serves both directions (a transform of the
+        // values with real and imaginary part exchanged is the backward one,
+        // exchanged), and the stages that have the same shape share one loop
+        // body: a quarter of the code of four unrolled stages, whose fetches
+        // stalled the passes (256^3 x 345 -> 305 us).
+        auto exchange = [](fxc &u) {
+            const long long t = u.x;
+            u.x = u.y;
+            u.y = t;
+        };
+        // the spectrum X[k], k = k0 + kstep i, of M values in `u`: Parseval
+        // sums, spectrum out, then the phase (or mask) and the exchange
+        auto spectrum = [&](auto &u, auto count, int k0, auto kstep) {
+            constexpr int M = decltype(count)::value, KS = decltype(kstep)::value;
+            const FxOut os(q + (N2 > 1 ? 2 : 0), bad, 1.0, false);
             if constexpr (MODE == MODE_FUSED || MODE == MODE_DIAG) {
                 if (red & RED_KIN) {
-                    const FxOut os(q, bad, 1.0, false);
                     T s2 = 0, s1 = 0;
 #pragma unroll
-                    for (int k = 0; k < N1; k++) kin(c[k], k, os, s2, s1);
+                    for (int i = 0; i < M; i++) kin(u[i], k0 + KS * i, os, s2, s1);
                     kin_add(s2, s1);
                 }
             }
-            if constexpr (MODE == MODE_FUSED) {
-                const int lim = kMask ? a.mask_lim[gg] : 0;
+            if constexpr (MODE == MODE_FWD) {
+                if (valid) {
 #pragma unroll
-                for (int k = 0; k < N1; k++) {
-                    if constexpr (kMask) {
-                        c[k] = (k < (N + 1) / 2 ? k : N - k) <= lim ? fx_quarter(c[k]) : fxc{0, 0};
-                    } else {
-                        c[k] = fx_cmul<false>(c[k], prow ? fxph[row * prow + k] : sph[k]);
-                    }
+                    for (int i = 0; i < M; i++) a.out[base + (uint32_t)(k0 + KS * i) * st] = os(u[i], (i & 1) == 0);
                 }
             }
-            if constexpr (MODE == MODE_FUSED || MODE == MODE_INV) dft<N1, +1>(c);
-            qo = q + (MODE == MODE_FUSED ? 2 + fxpe : 0);
-        } else {
-            // stage A: (k1, r) <- c[k1] w_n^{r k1} / 4
-            if constexpr (MODE != MODE_INV) {
+            if constexpr (MODE == MODE_FUSED && kMask) {
+                const int lim = a.mask_lim[gg];
+#pragma unroll
+                for (int i = 0; i < M; i++) {
+                    const int k = k0 + KS * i;
+                    u[i] = (k < (N + 1) / 2 ? k : N - k) <= lim ? fx_quarter(u[i]) : fxc{0, 0};
+                }
+            }
+        };
+        const int4 *phrow = prow ? fxph + row * prow : sph;
+        (void)phrow;
+        (void)spectrum;
+        using cN1 = std::integral_constant<int, N1>;
+        using cN2 = std::integral_constant<int, N2>;
+        using c1 = std::integral_constant<int, 1>;
+        constexpr bool kSpecOnly = MODE == MODE_FWD || MODE == MODE_DIAG;
+        int qo;  // the result's quantum
+        if constexpr (N2 == 1) {
+            // the whole line in this thread
+            if constexpr (MODE == MODE_INV) {
+#pragma unroll
+                for (int j = 0; j < N1; j++) exchange(c[j]);
+            }
+#pragma unroll 1
+            for (int it = MODE == MODE_INV ? 1 : 0; it < (kSpecOnly ? 1 : 2); it++) {
                 dft<N1, -1>(c);
+                if (it == 0) {
+                    spectrum(c, cN1{}, 0, c1{});
+                    if constexpr (MODE == MODE_FUSED) {
 #pragma unroll
-                for (int k1 = 0; k1 < N1; k1++) {
-                    const int m = k1 * N2 + r;
-                    sfx[sidx(m)] = k1 == 0 ? fx_quarter(c[0]) : fx_cmul<false>(c[k1], stw[m]);
-                }
-                line_sync();
-            }
-            // stage B: items k1 = r + P i
-            const FxOut os(q + 2, bad, 1.0, false);
-#pragma unroll
-            for (int i = 0; i < NI; i++) {
-                const int k1 = r + P * i;
-                fxc u[N2];
-                if constexpr (MODE == MODE_INV) {
-#pragma unroll
-                    for (int k2 = 0; k2 < N2; k2++) u[k2] = c[i * N2 + k2];
-                } else {
-#pragma unroll
-                    for (int rr = 0; rr < N2; rr++) u[rr] = sfx[sidx(k1 * N2 + rr)];
-                    dft<N2, -1>(u);  // u[k2] = X[k1 + N1 k2]
-                }
-                if constexpr (MODE == MODE_FWD) {
-                    if (valid) {
-#pragma unroll
-                        for (int k2 = 0; k2 < N2; k2++) a.out[base + (uint32_t)(k1 + N1 * k2) * st] = os(u[k2]);
-                    }
-                }
-                if constexpr (MODE == MODE_FUSED || MODE == MODE_DIAG) {
-                    if (red & RED_KIN) {
-                        T s2 = 0, s1 = 0;
-#pragma unroll
-                        for (int k2 = 0; k2 < N2; k2++) kin(u[k2], k1 + N1 * k2, os, s2, s1);
-                        kin_add(s2, s1);
-                    }
-                }
-                if constexpr (MODE == MODE_FUSED) {
-                    const int lim = kMask ? a.mask_lim[gg] : 0;
-#pragma unroll
-                    for (int k2 = 0; k2 < N2; k2++) {
-                        const int k = k1 + N1 * k2;
-                        if constexpr (kMask) {
-                            u[k2] = (k < (N + 1) / 2 ? k : N - k) <= lim ? fx_quarter(u[k2]) : fxc{0, 0};
-                        } else {
-                            u[k2] = fx_cmul<false>(u[k2], prow ? fxph[row * prow + k] : sph[k]);
+                        for (int j = 0; j < N1; j++) {
+                            if constexpr (!kMask) c[j] = fx_cmul(c[j], phrow[j]);
+                            exchange(c[j]);
                         }
                     }
                 }
-                if constexpr (MODE == MODE_FUSED || MODE == MODE_INV) {
-                    dft<N2, +1>(u);  // u[rr] = Z[k1][rr]
+            }
+            qo = q + (MODE == MODE_FUSED ? 2 + fxpe : 0);
+        } else if constexpr (N1 == N2) {
+            // stages A, B forward, B backward, C as one loop: every one
+            // transforms N1 values, all but the last multiply value j by entry
+            // j N2 + r of a table (twiddles, phase, twiddles), and A and B's
+            // backward part store what the next stage gathers, transposed
+            if constexpr (MODE == MODE_INV) {
 #pragma unroll
-                    for (int rr = 0; rr < N2; rr++)
-                        sfx[sidx(k1 * N2 + rr)] = rr == 0 ? fx_quarter(u[0]) : fx_cmul<true>(u[rr], stwB[rr * N1 + k1]);
+                for (int j = 0; j < N1; j++) exchange(c[j]);
+            }
+            const int oc = XL ? w * LS + r : r * W + w;                     // (j, r): column r
+            const int orow = XL ? w * LS + r * (N2 + 1) : r * N2 * W + w;   // (r, j): row r
+            constexpr int SC = XL ? N2 + 1 : N2 * W, SR = XL ? 1 : W;
+#pragma unroll 1
+            for (int it = MODE == MODE_INV ? 2 : 0; it < (kSpecOnly ? 2 : 4); it++) {
+                if (it & 1) {
+                    line_sync();
+                    const int off = it == 1 ? orow : oc, step = it == 1 ? SR : SC;
+#pragma unroll
+                    for (int j = 0; j < N1; j++) c[j] = sfx[off + j * step];
+                }
+                dft<N1, -1>(c);
+                if (it == 1) spectrum(c, cN1{}, r, cN2{});
+                if (it < 3 && !(it == 1 && (kSpecOnly || kMask))) {
+                    const int4 *tab = (it == 1 ? phrow : stw) + r;
+#pragma unroll
+                    for (int j = 0; j < N1; j++) c[j] = fx_cmul(c[j], tab[j * N2]);
+                }
+                if (it == 1) {
+#pragma unroll
+                    for (int j = 0; j < N1; j++) exchange(c[j]);
+                }
+                if (!(it & 1)) {
+                    const int off = it == 0 ? oc : orow, step = it == 0 ? SC : SR;
+#pragma unroll
+                    for (int j = 0; j < N1; j++) sfx[off + j * step] = c[j];
                 }
             }
-            if constexpr (MODE == MODE_FUSED || MODE == MODE_INV) {
-                line_sync();
-                // stage C
+            qo = q + (MODE == MODE_FUSED ? 6 + fxpe : 2);
+        } else {
+            // stages A and C share a loop body, B's two parts another
+#pragma unroll 1
+            for (int half = MODE == MODE_INV ? 1 : 0; half < 2; half++) {
+                if (half == 0 || MODE != MODE_INV) dft<N1, -1>(c);
+                if (half == 0) {
+                    // stage A: (k1, r) <- c[k1] w_n^{r k1} / 4
 #pragma unroll
-                for (int k1 = 0; k1 < N1; k1++) c[k1] = sfx[sidx(k1 * N2 + r)];
-                dft<N1, +1>(c);
+                    for (int k1 = 0; k1 < N1; k1++) sfx[sidx(k1 * N2 + r)] = fx_cmul(c[k1], stw[k1 * N2 + r]);
+                    line_sync();
+                }
+                if (half == 0 || MODE == MODE_INV) {
+                    // stage B: items k1 = r + P i (the spectrum of an INV pass
+                    // lies in c, so its items are unrolled)
+                    auto item = [&](int k1, auto fixed_item) {
+                        fxc u[N2];
+                        if constexpr (MODE == MODE_INV) {
+                            constexpr int I = decltype(fixed_item)::value;
+#pragma unroll
+                            for (int k2 = 0; k2 < N2; k2++) {
+                                u[k2] = c[I * N2 + k2];
+                                exchange(u[k2]);
+                            }
+                        } else {
+#pragma unroll
+                            for (int rr = 0; rr < N2; rr++) u[rr] = sfx[sidx(k1 * N2 + rr)];
+                        }
+#pragma unroll 1
+                        for (int d = MODE == MODE_INV ? 1 : 0; d < (kSpecOnly ? 1 : 2); d++) {
+                            dft<N2, -1>(u);
+                            if (d == 0) spectrum(u, cN2{}, k1, cN1{});
+                            if (!(d == 0 && (kSpecOnly || kMask))) {
+                                const int4 *tab = (d == 0 ? phrow : stwB) + k1;
+#pragma unroll
+                                for (int k2 = 0; k2 < N2; k2++) u[k2] = fx_cmul(u[k2], tab[N1 * k2]);
+                            }
+                            if (d == 0) {
+#pragma unroll
+                                for (int k2 = 0; k2 < N2; k2++) exchange(u[k2]);
+                            }
+                        }
+                        if constexpr (!kSpecOnly) {
+#pragma unroll
+                            for (int rr = 0; rr < N2; rr++) sfx[sidx(k1 * N2 + rr)] = u[rr];
+                        }
+                    };
+                    if constexpr (MODE == MODE_INV) {
+                        item(r, std::integral_constant<int, 0>{});
+                        if constexpr (NI > 1) item(r + P, std::integral_constant<int, 1>{});
+                        static_assert(NI <= 2, "two items per thread at most");
+                    } else {
+#pragma unroll 1
+                        for (int i = 0; i < NI; i++) item(r + P * i, c1{});
+                    }
+                    if constexpr (kSpecOnly) break;
+                    line_sync();
+#pragma unroll
+                    for (int k1 = 0; k1 < N1; k1++) c[k1] = sfx[sidx(k1 * N2 + r)];
+                }
+                if (MODE == MODE_INV) dft<N1, -1>(c);
             }
             qo = q + (MODE == MODE_FUSED ? 6 + fxpe : 2);
         }
-        if constexpr (MODE != MODE_DIAG && !(MODE == MODE_FWD && N2 > 1)) {
+        if constexpr (MODE == MODE_FUSED || MODE == MODE_INV) {
+#pragma unroll
+            for (int j = 0; j < N1; j++) exchange(c[j]);
+        }
+        if constexpr (MODE == MODE_FUSED || MODE == MODE_INV) {
             // 1/n of the inverse, and the deferred factor
-            int qv = MODE == MODE_FWD ? qo : qo - FxLog<N>::V;
+            int qv = qo - FxLog<N>::V;
             if constexpr (MODE == MODE_FUSED && kNL) {
                 if (fxnl) {
                     if constexpr (kAdj) {
                         if (a.pre_out && valid) {
                             const FxOut op(qv, bad, 1.0, false);
 #pragma unroll
-                            for (int j = 0; j < N1; j++) a.pre_out[base + (uint32_t)(r + N2 * j) * st] = op(c[j]);
+                            for (int j = 0; j < N1; j++) a.pre_out[base + (uint32_t)(r + N2 * j) * st] = op(c[j], (j & 1) == 0);
                         }
                     }
                     // the values are below 2^60 n / 64 (whole line in a
@@ -853,7 +936,7 @@ pass_kernel(const PassArgs<T> a)
             }
             const FxOut oc(qv, bad || vbad, (double)tscale, MODE == MODE_FUSED && tscaled);
 #pragma unroll
-            for (int j = 0; j < N1; j++) v[j] = oc(c[j]);
+            for (int j = 0; j < N1; j++) v[j] = oc(c[j], N == 256 || (j & 1) == 0);
         }
     } else if constexpr (kComp) {
         // compensated kinetic pass: the same stages on gridded two-float
@@ -1273,7 +1356,7 @@ pass_kernel(const PassArgs<T> a)
                 for (int j = 0; j < N1; j++) a.out[base + (uint32_t)(r + N2 * j) * st] = v[j];
             }
         }
-    } else if constexpr (MODE == MODE_FWD && N2 == 1) {
+    } else if constexpr (MODE == MODE_FWD && N2 == 1 && !kFix) {
         if (valid) {
 #pragma unroll
             for (int k = 0; k < N1; k++) a.out[base + (uint32_t)k * st] = v[k];

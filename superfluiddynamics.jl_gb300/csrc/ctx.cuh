@@ -62,7 +62,8 @@ struct gpss_ctx {
     void *tw[3] = {nullptr, nullptr, nullptr};  // per axis: register-kernel twiddles, or the generic pass's roots
     // axes whose lines the generic pass runs (not a power of two in [2, 256])
     bool gen[3] = {false, false, false};
-    GenPlan gplan[3] = {};
+    GenPlan gplan[3] = {};      // FP64
+    Gen32Plan gplan32[3] = {};  // FP32
     double *coord_dev[3] = {nullptr, nullptr, nullptr};
     std::vector<double> coord[3];
     double *partials = nullptr;
@@ -190,8 +191,13 @@ static int upload_fx(gpss_ctx *c, void **dev, const std::vector<int4> &t)
     CUDA_TRY(c, cudaMemcpy(*dev, t.data(), t.size() * sizeof(int4), cudaMemcpyHostToDevice));
     return GPSS_OK;
 }
-// does this axis run the register pass of an FP64 field (fixed-point tables)?
-static bool fx_axis(const gpss_ctx *c, int axis) { return c->precision == GPSS_FP64 && !c->gen[axis]; }
+// raw table bytes
+static int upload_bytes(gpss_ctx *c, void **dev, const void *data, size_t bytes)
+{
+    GPSS_TRY(dev_alloc(c, dev, bytes));
+    CUDA_TRY(c, cudaMemcpy(*dev, data, bytes, cudaMemcpyHostToDevice));
+    return GPSS_OK;
+}
 
 static void clear_graphs(gpss_ctx *c);
 
@@ -216,9 +222,11 @@ static int get_phase(gpss_ctx *c, int axis, double dtl, int imag, int fused, con
     const bool rot = c->omega != 0.0 && axis < 2 && c->ndim >= 2;
     const int64_t rows = rot ? (axis == 0 ? c->n[1] : c->n[0]) : 1;
     std::vector<ldouble> re((size_t)(n * rows)), im((size_t)(n * rows));
-    // fixed-point passes divide by n (a power of two) on the way out
-    const bool fx = fused && fx_axis(c, axis);
-    const ldouble inv_n = fused && !fx ? 1.0L / (ldouble)n : 1.0L;
+    // fused tables of FP64 fields are fixed point (their register passes divide
+    // by n, a power of two, on the way out; their generic passes want their
+    // spectrum's order)
+    const bool fx = fused && c->precision == GPSS_FP64, gen = fx && c->gen[axis];
+    const ldouble inv_n = fused && !(fx && !gen) ? 1.0L / (ldouble)n : 1.0L;
     for (int64_t r = 0; r < rows; r++) {
         const double cr = rot ? (axis == 0 ? c->coord[1][(size_t)r] : c->coord[0][(size_t)r]) : 0.0;
         for (int64_t k = 0; k < n; k++) {
@@ -236,10 +244,23 @@ static int get_phase(gpss_ctx *c, int axis, double dtl, int imag, int fused, con
             re[(size_t)(r * n + k)] = fr * inv_n;
             im[(size_t)(r * n + k)] = fi * inv_n;
         }
+        if (gen) {
+            std::vector<ldouble> tr((size_t)n), ti((size_t)n);
+            for (int64_t p = 0; p < n; p++) {
+                const int64_t k = gen_mode_at(c->gplan[axis], (int)p);
+                tr[(size_t)p] = re[(size_t)(r * n + k)];
+                ti[(size_t)p] = im[(size_t)(r * n + k)];
+            }
+            std::copy(tr.begin(), tr.end(), re.begin() + r * n);
+            std::copy(ti.begin(), ti.end(), im.begin() + r * n);
+        }
     }
     PhaseEntry e{axis, imag, fused, dtl, c->cD, c->omega, nullptr, rot ? (fx ? n : 2 * n) : 0};
-    if (fx) GPSS_TRY(upload_fx(c, &e.dev, fx_phase_table(re, im)));
-    else GPSS_TRY(upload_dw(c, &e.dev, re, im, rows, n));
+    if (fx) {
+        GPSS_TRY(upload_fx(c, &e.dev, fx_phase_table(re, im)));
+    } else {
+        GPSS_TRY(upload_dw(c, &e.dev, re, im, rows, n));
+    }
     if (c->phases.size() > 64) {  // bounded cache: drop the oldest
         clear_graphs(c);
         cudaStreamSynchronize(c->stream);
@@ -372,15 +393,15 @@ static void clear_vturns(gpss_ctx *c)
 }
 
 // the nonlinear flow N(dt) as the epilogue of a pass
-template <typename T> static int set_nl(gpss_ctx *c, int axis, PassArgs<T> &a, int mode, double dt)
+template <typename T> static int set_nl(gpss_ctx *c, PassArgs<T> &a, int mode, double dt)
 {
     a.nl_mode = mode;
     a.V = c->have_V ? (const T *)c->V : nullptr;
     a.nl_beta = c->beta;
     a.nl_dt = dt;
     a.nl_split = nl_split(c->beta, dt);
-    if (!fx_axis(c, axis) || mode != NL_REAL) return GPSS_OK;
-    // FP64 register pass: the flow in fixed point
+    if (c->precision != GPSS_FP64 || mode != NL_REAL) return GPSS_OK;
+    // FP64: the flow in fixed point
     if (!c->nl_tab) {
         std::vector<int4> t(FX_NL_TAB);
         for (int k = 0; k < FX_NL_TAB; k++) {
@@ -431,7 +452,11 @@ static bool any_generic(const gpss_ctx *c) { return c->gen[0] || c->gen[1] || c-
 
 template <typename T> static int blocks_for(gpss_ctx *c, int axis)
 {
-    if (c->gen[axis]) return (int)((c->total / c->n[axis] + c->gplan[axis].W - 1) / c->gplan[axis].W);
+    if (c->gen[axis]) {  // the smallest tile of the axis's kernels
+        const int W = sizeof(T) == 8 ? c->gplan[axis].lines()
+                                     : std::min(1 << c->gplan32[axis].lw, c->gplan32[axis].W);
+        return (int)((c->total / c->n[axis] + W - 1) / W);
+    }
     const int W = PassLauncher<T>::lines((int)c->n[axis], axis == 0);
     const int64_t nl = c->total / c->n[axis];
     return (int)((nl + W - 1) / W);
@@ -484,7 +509,7 @@ template <typename T> static int launch(gpss_ctx *c, int axis, int mode, const P
         return GPSS_OK;
     }
     if (c->gen[axis]) {
-        cudaError_t e = PassLauncher<T>::gen(mode, a, c->gplan[axis], c->stream);
+        cudaError_t e = PassLauncher<T>::gen(mode, a, c->gplan[axis], c->gplan32[axis], c->stream);
         if (e != cudaSuccess)
             return fail(c, GPSS_ECUDA, "generic pass launch (axis %d, n = %lld, mode %d): %s", axis,
                         (long long)c->n[axis], mode, cudaGetErrorString(e));
@@ -551,7 +576,7 @@ static int kinetic_fused(gpss_ctx *c, double dtl, int imag, bool nl, double dtnl
         }
         if (prescale && step == 0) a.scale = c->scale;
         const bool last = step == c->ndim - 1;
-        if (last && nl) GPSS_TRY(set_nl<T>(c, axis, a, imag ? NL_IMAG : NL_REAL, dtnl));
+        if (last && nl) GPSS_TRY(set_nl<T>(c, a, imag ? NL_IMAG : NL_REAL, dtnl));
         if (last) a.red |= red_last;
         if (a.red & RED_POINT) a.V = c->have_V ? (const T *)c->V : nullptr;
         if (diag_kin) {

@@ -99,7 +99,7 @@ static int imag_flow(gpss_ctx *c, double dtl, const void *in0, bool pre_nl, void
         const void *ph;
         GPSS_TRY(get_phase(c, axis, dtl, 1, 1, &ph, &a.prow));
         a.phase = (const vec2<T> *)ph;
-        if ((first && pre_nl) || (last && nl_last)) GPSS_TRY(set_nl<T>(c, axis, a, NL_NONE, dtnl));
+        if ((first && pre_nl) || (last && nl_last)) GPSS_TRY(set_nl<T>(c, a, NL_NONE, dtnl));
         if (first && pre_nl) {
             a.nl_pre = 1;
             a.scale = c->scale;
@@ -296,7 +296,7 @@ static int step_impl(gpss_ctx *c, int nsteps, int scheme, int imag, double dt, g
             c->pending_scale = lock;
         }
     } else if (imag && scheme == GPSS_STRANG && c->omega == 0.0 && !(c->flags & GPSS_FLAG_NOMERGE) &&
-               !any_generic(c)) {
+               (sizeof(T) == 8 || !any_generic(c))) {
         GPSS_TRY(imag_merged<T>(c, nsteps, dt));
     } else if (imag) {
         for (int s = 0; s < nsteps; s++) {
@@ -434,7 +434,6 @@ int gpss_create(gpss_ctx **out, int ndim, const int64_t *n, const double *lo, co
         c->gen[a] = !reg_line(n[a]);
         if (c->gen[a]) {
             gen_plan_radices((int)n[a], c->gplan[a]);
-            c->gplan[a].W = gen_tile_lines((int)n[a], precision == GPSS_FP32 ? 4 : 8);
         }
     }
     for (int a = 0; a < 3; a++) {
@@ -446,6 +445,13 @@ int gpss_create(gpss_ctx **out, int ndim, const int64_t *n, const double *lo, co
         c->total *= c->n[a];
         grid_coords(c->n[a], c->lo[a], c->hi[a], c->coord[a]);
     }
+    for (int a = 0; a < ndim; a++)
+        if (c->gen[a]) {
+            gen32_plan((int)n[a], c->gplan32[a]);
+            // (FP32 columns: at most 8, so that each has 16 threads for its sums)
+            c->gplan[a].lw = gen_tile_log((int)n[a], c->total / n[a], a == 0);
+            c->gplan32[a].lw = a == 0 ? c->gplan[a].lw : std::min(c->gplan[a].lw, 3);
+        }
     auto bail = [&](int rc) {
         g_create_error = c->err;
         gpss_destroy(c);
@@ -465,23 +471,28 @@ int gpss_create(gpss_ctx **out, int ndim, const int64_t *n, const double *lo, co
     // twiddles per axis, stage-A layout m = k1*N2 + r: exp(-2 pi i r k1 / n) as hi + lo
     for (int a = 0; a < ndim; a++) {
         const int64_t na = c->n[a];
-        std::vector<ldouble> re, im;
         if (c->gen[a]) {
-            // generic pass: the roots w_n^k = exp(-2 pi i k / n), k < n
-            re.resize((size_t)na);
-            im.resize((size_t)na);
-            for (int64_t k = 0; k < na; k++) {
-                ldouble cs, sn;
-                unit_root(k, na, &cs, &sn);
-                re[(size_t)k] = cs;
-                im[(size_t)k] = -sn;
+            if (precision == GPSS_FP64) {
+                const std::vector<unsigned char> t = gen_roots_table(c->gplan[a]);
+                rc = upload_bytes(c, &c->tw[a], t.data(), t.size());
+            } else {
+                // the roots w_n^k = exp(-2 pi i k / n), k < n
+                std::vector<ldouble> re((size_t)na), im((size_t)na);
+                for (int64_t k = 0; k < na; k++) {
+                    ldouble cs, sn;
+                    unit_root(k, na, &cs, &sn);
+                    re[(size_t)k] = cs;
+                    im[(size_t)k] = -sn;
+                }
+                rc = upload_dw(c, &c->tw[a], re, im, 1, na);
             }
-            if ((rc = upload_dw(c, &c->tw[a], re, im, 1, na))) return bail(rc);
+            if (rc) return bail(rc);
         } else {
             // two rows: stage-A order (k1*N2 + r) and stage-B order (r*N1 + k1)
+            std::vector<ldouble> re, im;
             twiddle_rows(na, precision == GPSS_FP64 ? 8 : 4, re, im);
-            if ((rc = fx_axis(c, a) ? upload_fx(c, &c->tw[a], fx_table(re, im))
-                                    : upload_dw(c, &c->tw[a], re, im, 2, na)))
+            if ((rc = precision == GPSS_FP64 ? upload_fx(c, &c->tw[a], fx_table(re, im))
+                                             : upload_dw(c, &c->tw[a], re, im, 2, na)))
                 return bail(rc);
         }
         if ((rc = dev_alloc(c, (void **)&c->coord_dev[a], sizeof(double) * (size_t)c->n[a]))) return bail(rc);
@@ -801,7 +812,7 @@ int gpss_time_pass(gpss_ctx *c, int axis, int mode, int reps, double dt, double 
             a.fin_status = c->status;
             CUDA_TRY(c, cudaMemsetAsync(c->status, 0, sizeof(int), c->stream));
         }
-        if (mode == 1) GPSS_TRY(set_nl<T>(c, axis, a, NL_REAL, dt));
+        if (mode == 1) GPSS_TRY(set_nl<T>(c, a, NL_REAL, dt));
         GPSS_TRY(launch<T>(c, axis, MODE_FUSED, a));  // warm-up
         CUDA_TRY(c, cudaEventRecord(c->ev[6], c->stream));
         for (int i = 0; i < reps; i++) GPSS_TRY(launch<T>(c, axis, MODE_FUSED, a));

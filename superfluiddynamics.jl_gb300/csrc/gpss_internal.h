@@ -3,10 +3,12 @@
 #include <cuda_runtime.h>
 #include <cmath>
 #include <cstdint>
+#include <cstring>
 #include <string>
 #include <vector>
 #include "pass_kernel.cuh"
 #include "pass_generic.cuh"
+#include "pass_generic32.cuh"
 
 namespace gpss {
 
@@ -139,6 +141,27 @@ inline void fx_turns(long double x, int64_t &m, int &e)
     e -= 62;
 }
 
+// The FP64 generic pass's tables: its roots w_n^k = exp(-2 pi i k / n), k < n, then the spectrum's order: mode
+// at each position, position of each mode
+inline std::vector<unsigned char> gen_roots_table(const GenPlan &p)
+{
+    const int n = p.n;
+    std::vector<long double> re((size_t)n), im((size_t)n);
+    std::vector<int> order((size_t)(2 * n));
+    for (int k = 0; k < n; k++) {
+        long double cs, sn;
+        unit_root(k, n, &cs, &sn);
+        re[(size_t)k] = cs;
+        im[(size_t)k] = -sn;
+        order[(size_t)k] = gen_mode_at(p, k);
+        order[(size_t)(n + order[(size_t)k])] = k;
+    }
+    std::vector<unsigned char> out((size_t)n * 16 + order.size() * sizeof(int));
+    std::memcpy(out.data(), fx_table(re, im).data(), (size_t)n * 16);
+    std::memcpy(out.data() + (size_t)n * 16, order.data(), order.size() * sizeof(int));
+    return out;
+}
+
 // pass launchers (pass_f32.cu / pass_f64.cu)
 cudaError_t launch_pass_f32(int mode, bool xl, int n, const PassArgs<float> &a, int blocks,
                             cudaStream_t s);
@@ -150,7 +173,7 @@ int pass_lines_per_cta_f64(int n, bool xl);
 cudaError_t launch_pipe_f32(bool xl, int n, const PassArgs<float> &a, int ntiles, cudaStream_t s);
 
 // the generic-length pass (pass_gen.cu)
-cudaError_t launch_gen_f32(int mode, const PassArgs<float> &a, const GenPlan &p, cudaStream_t s);
+cudaError_t launch_gen_f32(int mode, const PassArgs<float> &a, const Gen32Plan &p, cudaStream_t s);
 cudaError_t launch_gen_f64(int mode, const PassArgs<double> &a, const GenPlan &p, cudaStream_t s);
 
 template <typename T> struct PassLauncher;
@@ -162,7 +185,7 @@ template <> struct PassLauncher<float> {
     {
         return launch_pipe_f32(xl, n, a, ntiles, s);
     }
-    static cudaError_t gen(int mode, const PassArgs<float> &a, const GenPlan &p, cudaStream_t s)
+    static cudaError_t gen(int mode, const PassArgs<float> &a, const GenPlan &, const Gen32Plan &p, cudaStream_t s)
     {
         return launch_gen_f32(mode, a, p, s);
     }
@@ -172,23 +195,11 @@ template <> struct PassLauncher<double> {
                               cudaStream_t s) { return launch_pass_f64(mode, xl, n, a, blocks, s); }
     static int lines(int n, bool xl) { return pass_lines_per_cta_f64(n, xl); }
     static cudaError_t pipe(bool, int, const PassArgs<double> &, int, cudaStream_t) { return cudaErrorInvalidValue; }
-    static cudaError_t gen(int mode, const PassArgs<double> &a, const GenPlan &p, cudaStream_t s)
+    static cudaError_t gen(int mode, const PassArgs<double> &a, const GenPlan &p, const Gen32Plan &, cudaStream_t s)
     {
         return launch_gen_f64(mode, a, p, s);
     }
 };
-
-// Lines per tile of the generic pass: as many as fit about 96 KB of shared
-// memory (two buffers), at most 16 (FP32) / 8 (FP64) -- 128-byte rows of
-// adjacent columns for the y/z passes.
-inline int gen_tile_lines(int n, int precision_bytes)
-{
-    const size_t per_line = 2 * (size_t)n * 2 * (size_t)precision_bytes;
-    int W = (int)((96u * 1024u) / per_line);
-    const int cap = precision_bytes == 4 ? 16 : 8;
-    if (W > cap) W = cap;
-    return W < 1 ? 1 : W;
-}
 
 // Is a line of n cells taken by the register kernel (a power of two up to
 // 256)?  Otherwise the generic pass runs it.

@@ -504,6 +504,8 @@ int gpss_create(gpss_ctx **out, int ndim, const int64_t *n, const double *lo, co
         int b = precision == GPSS_FP32 ? blocks_for<float>(c, a) : blocks_for<double>(c, a);
         if (b > maxb) maxb = b;
     }
+    // (four cells per thread of 128: the FP64 passes of small fields)
+    if (precision == GPSS_FP64 && c->total <= QUAD_CELLS) maxb = std::max(maxb, (int)((c->total + 511) / 512));
     c->max_blocks = maxb;
     if ((rc = dev_alloc(c, (void **)&c->partials, sizeof(double) * RQ_COUNT * (size_t)maxb))) return bail(rc);
     if ((rc = dev_alloc(c, (void **)&c->sums, sizeof(double) * 4 * RQ_COUNT))) return bail(rc);

@@ -40,21 +40,27 @@ inline void unit_root(int64_t k, int64_t n, long double *cs, long double *sn)
 
 // The twiddles w_n^{r k1} = exp(-2 pi i r k1 / n) of a line of n cells in the
 // pass kernel's two orders: row 0 at m = k1*N2 + r (stage A), row 1 at
-// m = r*N1 + k1 (stage B), N1 of the passes of a precision (split_n1), N2 = n / N1.
+// m = r*N1 + k1 (stage B), N1 of the passes of a precision (split_n1), N2 = n / N1;
+// FP64: then row 2, w_n^k in natural order (the radix-4 stages of small fields).
 inline void twiddle_rows(int64_t n, int precision_bytes, std::vector<long double> &re, std::vector<long double> &im)
 {
     const int64_t N1 = split_n1(n, precision_bytes), N2 = n / N1;
-    re.assign((size_t)(2 * n), 0.0L);
-    im.assign((size_t)(2 * n), 0.0L);
+    const int64_t rows = precision_bytes == 8 ? 3 : 2;
+    re.assign((size_t)(rows * n), 0.0L);
+    im.assign((size_t)(rows * n), 0.0L);
+    std::vector<long double> cs((size_t)n), sn((size_t)n);
+    for (int64_t k = 0; k < n; k++) unit_root(k, n, &cs[(size_t)k], &sn[(size_t)k]);
+    auto put = [&](int64_t i, int64_t k) {
+        re[(size_t)i] = cs[(size_t)k];
+        im[(size_t)i] = -sn[(size_t)k];
+    };
     for (int64_t k1 = 0; k1 < N1; k1++)
         for (int64_t r = 0; r < N2; r++) {
-            long double cs, sn;
-            unit_root(r * k1, n, &cs, &sn);
-            re[(size_t)(k1 * N2 + r)] = cs;
-            im[(size_t)(k1 * N2 + r)] = -sn;
-            re[(size_t)(n + r * N1 + k1)] = cs;
-            im[(size_t)(n + r * N1 + k1)] = -sn;
+            put(k1 * N2 + r, r * k1);
+            put(n + r * N1 + k1, r * k1);
         }
+    if (rows == 3)
+        for (int64_t k = 0; k < n; k++) put(2 * n + k, k);
 }
 
 // Complex values in rows of n (long double) as double-word pairs of the field

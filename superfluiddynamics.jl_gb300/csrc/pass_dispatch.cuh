@@ -98,12 +98,27 @@ static cudaError_t launch_comp_mode(const PassArgs<float> &a, int blocks, cudaSt
     return launch_pass_inst<float, N, XL, MODE_FUSED, FEAT_COMP>(a, blocks, s);
 }
 
+template <typename T, int N, bool XL, int SIZE>
+static cudaError_t launch_pass_sized(int mode, const PassArgs<T> &a, int blocks, cudaStream_t s);
+
 template <typename T, int N, bool XL>
 static cudaError_t launch_pass_mode(int mode, const PassArgs<T> &a, int blocks, cudaStream_t s)
 {
     if constexpr (sizeof(T) == 4) {
         if (mode == MODE_FUSED && a.comp) return launch_comp_f32(XL, N, a, blocks, s);
     }
+    // small FP64 fields (lines of 16 cells and more): four cells per thread, see
+    // quad_pass for where the line lies
+    if constexpr (sizeof(T) == 8 && N >= 16) {
+        if ((int64_t)a.nlines * N <= QUAD_CELLS) return launch_pass_sized<T, N, XL, FEAT_SMALL>(mode, a, blocks, s);
+    }
+    return launch_pass_sized<T, N, XL, 0>(mode, a, blocks, s);
+}
+
+// SIZE: 0, or FEAT_SMALL of an FP64 pass
+template <typename T, int N, bool XL, int SIZE>
+static cudaError_t launch_pass_sized(int mode, const PassArgs<T> &a, int blocks, cudaStream_t s)
+{
     switch (mode) {
     case MODE_FUSED: {
         // the leanest instantiation that does everything the arguments ask for
@@ -113,14 +128,14 @@ static cudaError_t launch_pass_mode(int mode, const PassArgs<T> &a, int blocks, 
         const bool nl = a.nl_mode != NL_NONE || (a.red & RED_MASS);
         if (a.mask_lim) {
             if (diag || acc || adj || nl || a.nl_pre || a.dot_with) return cudaErrorInvalidValue;
-            return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_MASK>(a, blocks, s);
+            return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_MASK | SIZE>(a, blocks, s);
         }
         if (!a.phase) return cudaErrorInvalidValue;  // every other fused pass reads a phase table
         // the fixed-point nonlinear flow takes the field unscaled, and its table
         if (sizeof(T) == 8 && a.nl_mode == NL_REAL && (a.scale || !a.nl_fx.tab)) return cudaErrorInvalidValue;
         if (a.nl_pre || a.dot_with) {
             if (diag || acc || adj || a.nl_mode != NL_NONE) return cudaErrorInvalidValue;
-            return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_IMAGM>(a, blocks, s);
+            return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_IMAGM | SIZE>(a, blocks, s);
         }
         if constexpr (sizeof(T) == 4 && N >= 64) {
             if (a.plane_nl || a.plane_scale) {
@@ -136,8 +151,8 @@ static cudaError_t launch_pass_mode(int mode, const PassArgs<T> &a, int blocks, 
                 return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_TMA>(a, blocks, s);
             }
         }
-        if (diag || (acc && (adj || nl))) return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_ALL>(a, blocks, s);
-        if (acc) return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_ACC>(a, blocks, s);
+        if (diag || (acc && (adj || nl))) return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_ALL | SIZE>(a, blocks, s);
+        if (acc) return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_ACC | SIZE>(a, blocks, s);
         if constexpr (sizeof(T) == 4 && !XL && N >= 64) {
             // fewer default tiles than SMs: the 128-thread y/z instantiation
             if (blocks < sm_count()) {
@@ -149,15 +164,15 @@ static cudaError_t launch_pass_mode(int mode, const PassArgs<T> &a, int blocks, 
             }
         }
         if (adj) {
-            if (nl) return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_ADJ | FEAT_NL>(a, blocks, s);
-            return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_ADJ>(a, blocks, s);
+            if (nl) return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_ADJ | FEAT_NL | SIZE>(a, blocks, s);
+            return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_ADJ | SIZE>(a, blocks, s);
         }
-        if (nl) return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_NL>(a, blocks, s);
-        return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_NONE>(a, blocks, s);
+        if (nl) return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_NL | SIZE>(a, blocks, s);
+        return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_NONE | SIZE>(a, blocks, s);
     }
-    case MODE_FWD: return launch_pass_inst<T, N, XL, MODE_FWD>(a, blocks, s);
-    case MODE_INV: return launch_pass_inst<T, N, XL, MODE_INV>(a, blocks, s);
-    case MODE_DIAG: return launch_pass_inst<T, N, XL, MODE_DIAG>(a, blocks, s);
+    case MODE_FWD: return launch_pass_inst<T, N, XL, MODE_FWD, FEAT_ALL | SIZE>(a, blocks, s);
+    case MODE_INV: return launch_pass_inst<T, N, XL, MODE_INV, FEAT_ALL | SIZE>(a, blocks, s);
+    case MODE_DIAG: return launch_pass_inst<T, N, XL, MODE_DIAG, FEAT_ALL | SIZE>(a, blocks, s);
     default: return cudaErrorInvalidValue;
     }
 }

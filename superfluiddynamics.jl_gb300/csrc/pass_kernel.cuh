@@ -85,8 +85,9 @@ enum { NL_NONE = 0, NL_REAL = 1, NL_IMAG = 2 };
 //              of the last pass replaced by Re sum conj(dot_with) psi
 //   FEAT_ADJ   the discrete adjoint's epilogues (pre_out, adj_pre) without
 //              the energy sums (FEAT_DIAG includes them as well)
-//   FEAT_SMALL (launch shape, FP32 y/z lines) CTAs of 128 threads, for fields
-//              whose pass would otherwise have fewer tiles than SMs
+//   FEAT_SMALL (launch shape) FP32 y/z lines: CTAs of 128 threads, for fields
+//              whose pass would otherwise have fewer tiles than SMs; FP64
+//              lines: four cells per thread (quad_pass)
 //   FEAT_MASK  the 2/3 dealiasing filter in place of the phase: on the last
 //              axis of a spectrum already transformed along the others, keep
 //              the modes with |kk| <= mask_lim[line] (scaled by 1/n), zero the rest
@@ -294,6 +295,10 @@ template <typename T, bool XL, int FEAT = 0> struct PassGeom {
 #endif
 // FP64 passes hold every complex value as two 64-bit integers: 512 threads per
 // SM (128 registers, at most 100 bytes of spills in the largest instantiations).
+// (four cells per thread: 80 registers; 64 and 128 run the same within 3%)
+#ifndef GPSS_PASS_SM_THREADS_QUAD
+#define GPSS_PASS_SM_THREADS_QUAD 768
+#endif
 #ifndef GPSS_PASS_SM_THREADS_F64
 #define GPSS_PASS_SM_THREADS_F64 512
 #endif
@@ -313,7 +318,9 @@ template <typename T, bool XL, int MODE, int FEAT> struct PassOcc {
             ? GPSS_PASS_SM_THREADS_PLANE_XL_F32
             : GPSS_PASS_SM_THREADS_F32;
     static constexpr int MIN_BLOCKS =
-        (sizeof(T) == 4 ? SM_THREADS : GPSS_PASS_SM_THREADS_F64) / PassGeom<T, XL, FEAT>::THREADS;
+        (sizeof(T) == 4                ? SM_THREADS
+         : (FEAT & FEAT_SMALL) != 0 ? GPSS_PASS_SM_THREADS_QUAD
+                                       : GPSS_PASS_SM_THREADS_F64) / PassGeom<T, XL, FEAT>::THREADS;
 };
 
 // (FP64 lines of 32 and 64 cells split 8 x 4 and 8 x 8: twice the threads per
@@ -325,14 +332,28 @@ template <int N, int BYTES = 4> struct Split {
     static constexpr int N2 = N / N1;
 };
 
+// FP64 passes over small fields (FEAT_SMALL, lines of 16 cells and more): four
+// cells per thread in radix-4 stages instead of 8 or 16 -- N1 is then the values
+// per thread, N2 the threads per line, and a line's slots are padded by one in
+// four (its stages then meet in shared memory without bank conflicts).  A small
+// field's pass is one or two warps per scheduler, its time a thread's chain of
+// dependent integer operations: a quarter of the cells is a third of the time
+// (plain / nonlinear pass: 256^2 11.5 / 16.2 -> 4.7 / 5.8 us, 128^2 10.3 / 14.7
+// -> 4.0 / 5.0, 64^2 4.8 / 7.5 -> 3.3 / 4.4).  The extra stages' products and
+// exchanges cost a full chip 16 % (128^3 39.8 -> 46.8 us) to 34 % (256^3); at
+// 64^3 the two are even (6.8 / 10.0 against 6.9 / 9.5), which is the limit.
+constexpr int64_t QUAD_CELLS = 1 << 18;
+template <typename T, int N, int FEAT> constexpr bool quad_pass = sizeof(T) == 8 && (FEAT & FEAT_SMALL) != 0 && N >= 16;
+
 template <typename T, int N, bool XL, int FEAT = 0> struct PassShape {
-    static constexpr int N1 = Split<N, sizeof(T)>::N1;
-    static constexpr int N2 = Split<N, sizeof(T)>::N2;
+    static constexpr bool QUAD = quad_pass<T, N, FEAT>;
+    static constexpr int N1 = QUAD ? 4 : Split<N, sizeof(T)>::N1;
+    static constexpr int N2 = N / N1;
     static constexpr int P = N2;                       // threads per line
     static constexpr int THREADS = PassGeom<T, XL, FEAT>::THREADS;
     static constexpr int W = THREADS / P;              // lines per CTA
-    static constexpr int LS = N + N1 + N2;             // XL padded line stride (slots)
-    static constexpr int DATA1 = (N2 == 1) ? 0 : (XL ? W * LS : W * N);
+    static constexpr int LS = QUAD ? N + N / 4 : N + N1 + N2;  // XL padded line stride (slots)
+    static constexpr int DATA1 = (N2 == 1) ? 0 : (XL || QUAD ? W * LS : W * N);
     // compensated passes hold (hi, lo) of a value in one 16-byte slot: DATA1
     // such slots, the size of two value arrays (one 128-bit shared-memory
     // access per value and exchange instead of two 64-bit ones: 256^3 y pass
@@ -344,7 +365,8 @@ template <typename T, int N, bool XL, int FEAT = 0> struct PassShape {
     static constexpr int STAGE = TMA ? W * N : 0;
     // w_n^{r k1} at k1*N2 + r (stage A) and at r*N1 + k1 (stage B) are the same
     // table when N1 == N2: then only one is held
-    static constexpr bool TWB = N1 != N2;
+    // (FP64 radix-4 stages: the roots of unity in natural order instead)
+    static constexpr bool TWB = N1 != N2 && !QUAD;
     // tables: hi and lo (FP32), or one 16-byte fixed-point constant (FP64)
     // and, where the pass may carry the nonlinear flow, its roots of unity
     static constexpr int NLTAB = sizeof(T) == 8 && (FEAT & FEAT_NL) != 0 ? FX_NL_TAB : 0;
@@ -500,7 +522,7 @@ pass_kernel(const PassArgs<T> a)
     for (int i = tid; i < N; i += THREADS) {
         if constexpr (kFix) {
             const int4 *ft = reinterpret_cast<const int4 *>(a.tw);
-            stw[i] = ft[i];
+            stw[i] = ft[S::QUAD ? 2 * N + i : i];
             if (S::TWB) stwB[i] = ft[N + i];
             if (MODE == MODE_FUSED && !kMask && prow == 0) sph[i] = fxph[i];
         } else {
@@ -525,7 +547,8 @@ pass_kernel(const PassArgs<T> a)
     const uint32_t st = XL ? 1u : (uint32_t)a.stride;
 
     auto sidx = [&](int q) -> int {
-        if constexpr (XL) return w * LS + q + q / N2;
+        if constexpr (S::QUAD) return XL ? w * LS + q + q / 4 : (q + q / 4) * W + w;
+        else if constexpr (XL) return w * LS + q + q / N2;
         else return q * W + w;
     };
 
@@ -568,9 +591,9 @@ pass_kernel(const PassArgs<T> a)
     // (P divides 32) and only they touch the line's shared-memory slots, so
     // the exchanges between stages need only a warp barrier.  COL lines span
     // the CTA (lane stride W).
-    static_assert(!XL || 32 % P == 0, "an XL line must not straddle warps");
+    static_assert(!XL || 32 % P == 0 || S::QUAD, "an XL line must not straddle warps");
     auto line_sync = [] {
-        if constexpr (XL) __syncwarp();
+        if constexpr (XL && P <= 32) __syncwarp();
         else __syncthreads();
     };
     __syncthreads();  // tables ready
@@ -660,7 +683,25 @@ pass_kernel(const PassArgs<T> a)
         // FP64 field: the same stages on 64-bit fixed-point values.  The tile's
         // lines each take their quantum from their largest component.
         constexpr int NI = N1 / N2;
-        if constexpr (MODE == MODE_INV) {
+        // radix-4 stages: the natural-order mode of value i of this thread, whose
+        // positions 4 r + i follow the digits of the stages (4, 4, .. and a last
+        // 2 where log2 N is odd)
+        constexpr bool kQuad = S::QUAD, kOdd = kQuad && FxLog<N>::V % 2 != 0;
+        auto quad_mode = [&](int i) {
+            int pos = 4 * r + i, k = 0, scale = 1;
+#pragma unroll
+            for (int m = N / 4; m >= 1; m /= 4) {
+                k += scale * ((pos / m) & 3);
+                scale *= 4;
+            }
+            if constexpr (kOdd) k += scale * (pos & 1);
+            return k;
+        };
+        (void)quad_mode;
+        if constexpr (MODE == MODE_INV && kQuad) {
+#pragma unroll
+            for (int i = 0; i < N1; i++) v[i] = a.in[base + (uint32_t)quad_mode(i) * st];
+        } else if constexpr (MODE == MODE_INV) {
 #pragma unroll
             for (int i = 0; i < NI; i++)
 #pragma unroll
@@ -670,7 +711,7 @@ pass_kernel(const PassArgs<T> a)
         int word = fx_max_word<N1>(v);
         if constexpr (XL) {
 #pragma unroll
-            for (int o = P / 2; o > 0; o >>= 1) word = max(word, __shfl_xor_sync(0xffffffffu, word, o));
+            for (int o = (P < 32 ? P : 32) / 2; o > 0; o >>= 1) word = max(word, __shfl_xor_sync(0xffffffffu, word, o));
         } else {
 #pragma unroll
             for (int o = 16; o >= W; o >>= 1) word = max(word, __shfl_xor_sync(0xffffffffu, word, o));
@@ -679,39 +720,44 @@ pass_kernel(const PassArgs<T> a)
         float n2 = fx_norm2<N1>(v, ref);
         if constexpr (XL) {
 #pragma unroll
-            for (int o = P / 2; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+            for (int o = (P < 32 ? P : 32) / 2; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
         } else {
 #pragma unroll
             for (int o = 16; o >= W; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
-            if constexpr (P > 1) {
-                // columns: so far over the lanes of a warp that hold the same
-                // column, now across the CTA.  No further barrier is needed:
+        }
+        {
+            if constexpr (XL ? P > 32 : P > 1) {
+                // so far over the lanes of a warp that hold the same line, now
+                // across the CTA.  No further barrier is needed:
                 // every thread reads the sums before the barrier after stage
                 // A, and the next tile writes them after the one before stage
                 // C (or its top one)
                 __shared__ int sword[THREADS];
                 __shared__ float snorm[THREADS];
-                constexpr int G = W < 32 ? THREADS / 32 : P;
-                const int slot = W < 32 ? (tid >> 5) * W + w : tid;
-                if (W >= 32 || (tid & 31) < W) {
+                constexpr int G = XL ? P / 32 : W < 32 ? THREADS / 32 : P;
+                const int slot = XL ? tid >> 5 : W < 32 ? (tid >> 5) * W + w : tid;
+                if ((XL ? (tid & 31) == 0 : W >= 32) || (!XL && (tid & 31) < W)) {
                     sword[slot] = word;
                     snorm[slot] = n2;
                 }
                 __syncthreads();
+                auto part = [&](int i) { return XL ? w * G + i : i * W + w; };
                 word = 0;
 #pragma unroll
-                for (int i = 0; i < G; i++) word = max(word, sword[i * W + w]);
+                for (int i = 0; i < G; i++) word = max(word, sword[part(i)]);
                 ref = fx_ref(word);
                 n2 = 0.f;
 #pragma unroll
                 for (int i = 0; i < G; i++) {
-                    const int d = max(fx_ref(sword[i * W + w]) - ref, -50);
-                    n2 = fmaf(snorm[i * W + w], __int_as_float((127 + 2 * d) << 23), n2);
+                    const int d = max(fx_ref(sword[part(i)]) - ref, -50);
+                    n2 = fmaf(snorm[part(i)], __int_as_float((127 + 2 * d) << 23), n2);
                 }
             }
         }
         const bool bad = word >= 0x7ff00000;
-        const int q = fx_quantum(ref, n2);
+        // (radix-4 stages double the modulus where others take it to 4 times
+        // the norm: one bit more)
+        const int q = kQuad ? max(fx_quantum(ref, n2) - 1, -1020) : fx_quantum(ref, n2);
         fxc c[N1];
 #pragma unroll
         for (int j = 0; j < N1; j++) {
@@ -779,7 +825,102 @@ pass_kernel(const PassArgs<T> a)
         using c1 = std::integral_constant<int, 1>;
         constexpr bool kSpecOnly = MODE == MODE_FWD || MODE == MODE_DIAG;
         int qo;  // the result's quantum
-        if constexpr (N2 == 1) {
+        if constexpr (kQuad) {
+            // Four values per thread, in place: forward stages of radix 4 with
+            // M = N/4, N/16, .. cells between a butterfly's values (decimation in
+            // frequency), the last one (M = 1; two radix-2 butterflies where
+            // log2 N is odd), the phase, and the mirror image back.  Products
+            // divide by 4 and are doubled, so that every stage's values fill
+            // the same bits.
+            auto doubled = [](fxc u) { return fxc{u.x + u.x, u.y + u.y}; };
+            auto product = [&](fxc u, const int4 &t) { return doubled(fx_cmul(u, t)); };
+            auto halved = [](fxc u) { return fxc{(u.x + 1) >> 1, (u.y + 1) >> 1}; };
+            auto slot0 = [&](int M, int &t) {  // the butterfly's first position, its root's index
+                const int j = r & (M - 1);
+                t = j * (N / 4 / M);
+                return (r - j) * 4 + j;
+            };
+            auto last = [&]() {
+                if constexpr (kOdd) {
+                    dft<2, -1>(c);
+                    dft<2, -1>(c + 2);
+                } else {
+                    dft<4, -1>(c);
+                }
+            };
+            constexpr int kLastM = kOdd ? 2 : 4;  // the smallest M above 1
+            constexpr int kF = kOdd ? (FxLog<N>::V - 1) / 2 : FxLog<N>::V / 2 - 1;  // stages above it
+            if constexpr (MODE != MODE_INV) {
+#pragma unroll 1
+                for (int M = N / 4; M >= kLastM; M >>= 2) {
+                    int t;
+                    const int p0 = slot0(M, t);
+                    if (M < N / 4) {
+                        line_sync();
+#pragma unroll
+                        for (int i = 0; i < 4; i++) c[i] = sfx[sidx(p0 + i * M)];
+                    }
+                    dft<4, -1>(c);
+                    c[0] = halved(c[0]);
+#pragma unroll
+                    for (int i = 1; i < 4; i++) c[i] = product(c[i], stw[i * t]);
+#pragma unroll
+                    for (int i = 0; i < 4; i++) sfx[sidx(p0 + i * M)] = c[i];
+                }
+                line_sync();
+#pragma unroll
+                for (int i = 0; i < 4; i++) c[i] = sfx[sidx(4 * r + i)];
+                last();
+                const FxOut os(q + kF, bad, 1.0, false);
+                if constexpr (MODE == MODE_FUSED || MODE == MODE_DIAG) {
+                    if (red & RED_KIN) {
+                        T s2 = 0, s1 = 0;
+#pragma unroll
+                        for (int i = 0; i < 4; i++) kin(c[i], quad_mode(i), os, s2, s1);
+                        kin_add(s2, s1);
+                    }
+                }
+                if constexpr (MODE == MODE_FWD) {
+                    if (valid) {
+#pragma unroll
+                        for (int i = 0; i < 4; i++) a.out[base + (uint32_t)quad_mode(i) * st] = os(c[i], false);
+                    }
+                }
+                if constexpr (MODE == MODE_FUSED) {
+                    const int lim = kMask ? a.mask_lim[gg] : 0;
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const int k = quad_mode(i);
+                        if constexpr (kMask) c[i] = (k < (N + 1) / 2 ? k : N - k) <= lim ? halved(c[i]) : fxc{0, 0};
+                        else c[i] = product(c[i], phrow[k]);
+                    }
+                }
+            }
+            if constexpr (!kSpecOnly) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) exchange(c[i]);
+                last();
+#pragma unroll
+                for (int i = 0; i < 4; i++) sfx[sidx(4 * r + i)] = c[i];
+#pragma unroll 1
+                for (int M = kLastM; M <= N / 4; M <<= 2) {
+                    int t;
+                    const int p0 = slot0(M, t);
+                    line_sync();
+#pragma unroll
+                    for (int i = 0; i < 4; i++) c[i] = sfx[sidx(p0 + i * M)];
+                    c[0] = halved(c[0]);
+#pragma unroll
+                    for (int i = 1; i < 4; i++) c[i] = product(c[i], stw[i * t]);
+                    dft<4, -1>(c);
+                    if (M < N / 4) {
+#pragma unroll
+                        for (int i = 0; i < 4; i++) sfx[sidx(p0 + i * M)] = c[i];
+                    }
+                }
+            }
+            qo = q + (MODE == MODE_FUSED ? 2 * kF + 1 + fxpe : kF);
+        } else if constexpr (N2 == 1) {
             // the whole line in this thread
             if constexpr (MODE == MODE_INV) {
 #pragma unroll
@@ -919,7 +1060,8 @@ pass_kernel(const PassArgs<T> a)
                     }
                     // the values are below 2^60 n / 64 (whole line in a
                     // thread: n / 4): shorter lines have room for more bits
-                    constexpr int KS = 2 - (FxLog<N>::V - (N2 > 1 ? 6 : 2));
+                    // (radix-4 stages: below 2^62, or 2^61 where log2 N is odd)
+                    constexpr int KS = kQuad ? (kOdd ? 1 : 0) : 2 - (FxLog<N>::V - (N2 > 1 ? 6 : 2));
                     qv -= KS;
                     const int sh = 190 + 2 * qv + a.nl_fx.ge;
                     const int lsh = min(max(sh, 0), 63), rsh = min(max(-sh, 0), 63);
@@ -936,7 +1078,7 @@ pass_kernel(const PassArgs<T> a)
             }
             const FxOut oc(qv, bad || vbad, (double)tscale, MODE == MODE_FUSED && tscaled);
 #pragma unroll
-            for (int j = 0; j < N1; j++) v[j] = oc(c[j], N == 256 || (j & 1) == 0);
+            for (int j = 0; j < N1; j++) v[j] = oc(c[j], !kQuad && (N == 256 || (j & 1) == 0));
         }
     } else if constexpr (kComp) {
         // compensated kinetic pass: the same stages on gridded two-float

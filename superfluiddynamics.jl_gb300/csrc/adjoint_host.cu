@@ -51,7 +51,7 @@ static int adj_group(gpss_ctx *c, void *buf, double dtl, bool reverse, bool nl, 
         // stay bitwise those of the forward)
         a.comp = sizeof(T) == 4 && (c->flags & GPSS_FLAG_COMPENSATED) != 0;
         if (step == c->ndim - 1 && (nl || adj_pre)) {
-            GPSS_TRY(set_nl<T>(c, a, nl ? NL_REAL : NL_NONE, dtnl));
+            GPSS_TRY(set_nl<T>(c, a, nl ? NL_REAL : NL_NONE, dtnl, true));
             if (nl) {
                 a.pre_out = (vec2<T> *)pre_out;
             } else {

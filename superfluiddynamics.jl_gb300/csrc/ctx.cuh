@@ -392,32 +392,42 @@ static void clear_vturns(gpss_ctx *c)
     c->vturns.clear();
 }
 
-// the nonlinear flow N(dt) as the epilogue of a pass
-template <typename T> static int set_nl(gpss_ctx *c, PassArgs<T> &a, int mode, double dt)
+// the nonlinear flow N(dt) of a pass: its epilogue (mode), or with NL_NONE the
+// constants of a prologue (imaginary time) or of the flow's adjoint (real_time)
+template <typename T> static int set_nl(gpss_ctx *c, PassArgs<T> &a, int mode, double dt, bool real_time)
 {
     a.nl_mode = mode;
     a.V = c->have_V ? (const T *)c->V : nullptr;
     a.nl_beta = c->beta;
     a.nl_dt = dt;
     a.nl_split = nl_split(c->beta, dt);
-    if (c->precision != GPSS_FP64 || mode != NL_REAL) return GPSS_OK;
-    // FP64: the flow in fixed point
+    if (c->precision != GPSS_FP64) return GPSS_OK;
+    // FP64: fixed point, see fft_fix.cuh
     if (!c->nl_tab) {
-        std::vector<int4> t(FX_NL_TAB);
-        for (int k = 0; k < FX_NL_TAB; k++) {
-            ldouble cs, sn;
-            unit_root(k, FX_NL_TAB, &cs, &sn);
-            t[(size_t)k] = fx_const(cs, sn);
-        }
-        GPSS_TRY(upload_fx(c, &c->nl_tab, t));
+        // the same for every context: made once per process
+        static const std::vector<int4> table = [] {
+            std::vector<int4> t((size_t)(FX_NL_TAB + FX_NL_TAB / 2));
+            long long pow2[FX_NL_TAB];
+            for (int k = 0; k < FX_NL_TAB; k++) {
+                ldouble cs, sn;
+                unit_root(k, FX_NL_TAB, &cs, &sn);
+                t[(size_t)k] = fx_const(cs, sn);
+                pow2[k] = llroundl(ldexpl(exp2l((ldouble)k / FX_NL_TAB), 61));
+            }
+            std::memcpy(&t[FX_NL_TAB], pow2, sizeof(pow2));
+            return t;
+        }();
+        GPSS_TRY(upload_fx(c, &c->nl_tab, table));
     }
+    a.nl_fx.tab = (const int4 *)c->nl_tab;
+    a.nl_fx.tab2 = (const long long *)(a.nl_fx.tab + FX_NL_TAB);
+    if (!real_time) return GPSS_OK;
     int64_t m;
     int e;
     fx_turns((ldouble)c->beta * (ldouble)dt, m, e);
     a.nl_fx.gl = (int)(uint32_t)m;
     a.nl_fx.gh = (int)((m - (int64_t)a.nl_fx.gl) >> 32);
     a.nl_fx.ge = e;
-    a.nl_fx.tab = (const int4 *)c->nl_tab;
     if (c->have_V) {
         if (!c->vbad) {
             GPSS_TRY(dev_alloc(c, (void **)&c->vbad, sizeof(int)));
@@ -576,7 +586,7 @@ static int kinetic_fused(gpss_ctx *c, double dtl, int imag, bool nl, double dtnl
         }
         if (prescale && step == 0) a.scale = c->scale;
         const bool last = step == c->ndim - 1;
-        if (last && nl) GPSS_TRY(set_nl<T>(c, a, imag ? NL_IMAG : NL_REAL, dtnl));
+        if (last && nl) GPSS_TRY(set_nl<T>(c, a, imag ? NL_IMAG : NL_REAL, dtnl, !imag));
         if (last) a.red |= red_last;
         if (a.red & RED_POINT) a.V = c->have_V ? (const T *)c->V : nullptr;
         if (diag_kin) {

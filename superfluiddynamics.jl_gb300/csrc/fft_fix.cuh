@@ -204,6 +204,22 @@ __device__ __forceinline__ long long fx_from(double x, int s0)
     return ((((long long)(m >> s)) ^ sg) - sg + 1) >> 1;
 }
 
+// v 2^q in FP64 by integer operations, |q| <= 900
+__device__ __forceinline__ double fx_double(long long v, int q)
+{
+    const int sg = (int)(v >> 63);
+    const unsigned long long m = (unsigned long long)((v ^ (long long)sg) - (long long)sg);
+    const unsigned mh = (unsigned)(m >> 32), ml = (unsigned)m;
+    const bool small = mh == 0;
+    const int z = __clz((int)(small ? ml : mh));
+    const unsigned nh = small ? ml << (z & 31) : __funnelshift_l(ml, mh, z);
+    const unsigned nl = small ? 0u : ml << z;
+    // the top bit, at 63, becomes the significand's implicit one
+    const unsigned lo = __funnelshift_r(nl, nh, 11), r = lo + ((nl >> 10) & 1u);
+    const unsigned e = (unsigned)((1023 + 62 + q - z - (small ? 32 : 0)) << 20) | ((unsigned)sg & 0x80000000u);
+    const unsigned hi = (nh >> 11) + e + (r < lo ? 1u : 0u);
+    return m == 0 ? 0.0 : __hiloint2double((int)hi, (int)r);
+}
 // ---- the nonlinear flow of real time on fixed-point values ----
 //
 // psi <- exp(-i theta) psi with theta = (V + beta |psi|^2) dt in turns, as a
@@ -222,6 +238,7 @@ struct FxNlArgs {
     const long long *vturn;  // V dt / (2 pi) per cell, 2^64 to a turn; nullable
     const int *vbad;         // nonzero: V holds NaN or infinity; nullable
     const int4 *tab;         // exp(2 pi i k / 128), k < 128, as table constants
+    const long long *tab2;   // 2^(k / 128) 2^61, k < 128 (imaginary time)
 };
 // series of cos and sin of (pi / 128) u, |u| <= 1, in z = u^2: Taylor
 // coefficients times 4 per power of z (a product by z comes out as z / 4)
@@ -231,19 +248,9 @@ constexpr int FX_C6 = 0x155d3c7e;
 constexpr long long FX_S1 = 0x6487ed5110b4612LL, FX_S3 = 0xa55de7312df3LL;
 constexpr int FX_S5 = 0x519af19e, FX_S7 = 0x132d3;
 
-// One cell: c of modulus at most 2^62; theta = |c|^2 2^-62 (gh 2^32 + gl) 2^-64
-// shifted left by lsh and right by rsh, plus vt.  Returns exp(-i theta) c / 4.
-__device__ __forceinline__ fxc fx_nl_real(fxc c, long long vt, int gh, int gl, int lsh, int rsh, const int4 *tab)
+// exp(2 pi i th / 2^64), 2^62 times its components
+__device__ __forceinline__ fxc fx_expi(long long th, const int4 *tab)
 {
-    int xh, xl, yh, yl;
-    fx_split(c.x, xh, xl);
-    fx_split(c.y, yh, yl);
-    // the squares of the low halves, left out, are 2/3 of a unit on average
-    constexpr long long kX = (1LL << 28) + (2LL << 29) / 3;
-    const long long S = fx_madw(xh, xh, fx_madw(yh, yh, 0));
-    const long long X = fx_madw(xl, xh, fx_madw(yl, yh, kX));
-    const long long rho = (S << 2) + (X >> 29);
-    const long long th = ((fx_rmul(rho, gh, gl) << lsh) >> rsh) + vt;
     const unsigned k = (unsigned)((unsigned long long)(th + (1LL << 56)) >> 57);
     const long long u = (long long)((unsigned long long)th << 6) - ((long long)((unsigned long long)k << 63));
     // u = 2^62 times the remainder over a 256th of a turn: th - k 2^57, times 64
@@ -267,6 +274,23 @@ __device__ __forceinline__ fxc fx_nl_real(fxc c, long long vt, int gh, int gl, i
     fxc f = fx_cmul(fxc{co, si}, tab[k & (FX_NL_TAB - 1)]);
     f.x <<= 2;
     f.y <<= 2;
+    return f;
+}
+
+// One cell: c of modulus at most 2^62; theta = |c|^2 2^-62 (gh 2^32 + gl) 2^-64
+// shifted left by lsh and right by rsh, plus vt.  Returns exp(-i theta) c / 4.
+__device__ __forceinline__ fxc fx_nl_real(fxc c, long long vt, int gh, int gl, int lsh, int rsh, const int4 *tab)
+{
+    int xh, xl, yh, yl;
+    fx_split(c.x, xh, xl);
+    fx_split(c.y, yh, yl);
+    // the squares of the low halves, left out, are 2/3 of a unit on average
+    constexpr long long kX = (1LL << 28) + (2LL << 29) / 3;
+    const long long S = fx_madw(xh, xh, fx_madw(yh, yh, 0));
+    const long long X = fx_madw(xl, xh, fx_madw(yl, yh, kX));
+    const long long rho = (S << 2) + (X >> 29);
+    const long long th = ((fx_rmul(rho, gh, gl) << lsh) >> rsh) + vt;
+    const fxc f = fx_expi(th, tab);
     // c conj(f) / 4 (run-time constants are negated whole, not by halves: a
     // low half of -2^31 has no negative)
     int fh, fl, gh2, gl2, nh, nl;
@@ -279,6 +303,64 @@ __device__ __forceinline__ fxc fx_nl_real(fxc c, long long vt, int gh, int gl, i
     o.y = fx_fold(fx_madw(yh, fh, fx_madw(xh, nh, FX_S0)),
                   fx_madw(yl, fh, fx_madw(xl, nh, fx_madw(yh, fl, fx_madw(xh, nl, FX_X0)))));
     return o;
+}
+
+// theta / (2 pi) of rho = |psi|^2 >= 0 in FP64 (without the potential's part), 2^64
+// to a turn: the significand of rho times beta dt / (2 pi), at the place of the
+// exponents
+__device__ __forceinline__ long long fx_theta(double rho, int gh, int gl, int ge)
+{
+    const int hi = __double2hiint(rho);
+    const unsigned lo = (unsigned)__double2loint(rho);
+    const int e = (hi >> 20) & 0x7ff;
+    const unsigned mh = (__funnelshift_l(lo, (unsigned)hi, 10) & 0x3fffffffu) | 0x40000000u;
+    const long long m = (long long)(((unsigned long long)mh << 32) | (unsigned long long)(lo << 10));
+    const int sh = e ? e + ge - 957 : -63;  // 0 and denormals: 0
+    return (fx_rmul(m, gh, gl) << min(max(sh, 0), 63)) >> min(max(-sh, 0), 63);
+}
+
+// ---- 2^-x for FP64 x on the integer pipes (the flow of imaginary time) ----
+//
+// -x as a 52-bit fraction below an 11-bit integer; the nearest 128th from a
+// table, the rest r (at most 1/256) from the series of 2^r to 2^-60, the integer
+// as the exponent: an FP64 value off by its last rounding and the 2^-53 of x's.
+// 17 multiply-adds, where FP64 exp is some 20 operations at a 14th of their
+// rate (128^3 imaginary-time x pass 151 -> 92 us).
+constexpr long long FX_E1 = 0x2c5c85fdf473de7LL, FX_E2 = 0x3d7f7bff058b2LL, FX_E3 = 0x38d611ae094LL, FX_E4 = 0x276556df7LL;
+constexpr int FX_E5 = 0x15d87fe, FX_E6 = 0xa185;
+__device__ __forceinline__ double fx_exp2neg(double x, const long long *tab2)
+{
+    const int hi = __double2hiint(x);
+    const unsigned lo = (unsigned)__double2loint(x);
+    const int ex = (hi >> 20) & 0x7ff;
+    const unsigned mh = (__funnelshift_l(lo, (unsigned)hi, 10) & 0x3fffffffu) | 0x40000000u;
+    const unsigned long long m = ((unsigned long long)mh << 32) | (unsigned long long)(lo << 10);
+    // round(-x 2^52): |x| below 2^10 (beyond: 0, infinity or NaN, below)
+    const long long sg = ~(long long)(hi >> 31);
+    const long long E = ((((long long)(m >> (min(max(1032 - ex, 0), 63)))) ^ sg) - sg + 1) >> 1;
+    const int k7 = (int)((E + (1LL << 44)) >> 45);  // nearest 128th
+    const long long u = (E - ((long long)k7 << 45)) << 18;  // 2^62 times the remainder over 1/256
+    const int uh = (int)(u >> 32);
+    const long long t4 = FX_E4 + (long long)__mulhi(uh, FX_E5 + __mulhi(uh, FX_E6));
+    int ch, cl;
+    fx_split(t4, ch, cl);
+    const long long t3 = FX_E3 + fx_rmul(u, ch, cl);
+    fx_split(t3, ch, cl);
+    const long long t2 = FX_E2 + fx_rmul(u, ch, cl);
+    fx_split(t2, ch, cl);
+    const long long t1 = FX_E1 + fx_rmul(u, ch, cl);
+    fx_split(t1, ch, cl);
+    const long long p = fx_rmul(u, ch, cl);  // 2^64 (2^r - 1)
+    fx_split(p, ch, cl);
+    const long long T = tab2[k7 & 127];
+    const unsigned long long v = (unsigned long long)(T + fx_rmul(T, ch, cl));  // top bit 60 or 61
+    const int z = 2 + (int)((v >> 61) ^ 1u);  // leading zeros
+    const int e = 1024 - z + (k7 >> 7);  // the biased exponent less one: the top bit, below, adds it
+    const unsigned long long n = v << z;
+    const unsigned long long bits = ((unsigned long long)(unsigned)e << 52) + (n >> 11) + ((n >> 10) & 1u);
+    double r = e < 0 ? 0.0 : __longlong_as_double((long long)bits);
+    if (ex > 1032) r = hi < 0 ? __longlong_as_double(0x7ff0000000000000LL) : 0.0;
+    return x != x ? x : r;
 }
 
 // Leaving fixed point: an integer v times 2^q as the FP64 nearest to it, in two
@@ -309,25 +391,10 @@ struct FxOut {
         const double l = __hiloint2double(0x43300000 + qc * (1 << 20), (int)v);
         return (h - k) + l;
     }
-    __device__ __forceinline__ double integer(long long v) const
-    {
-        const int sg = (int)(v >> 63);
-        const unsigned long long m = (unsigned long long)((v ^ (long long)sg) - (long long)sg);
-        const unsigned mh = (unsigned)(m >> 32), ml = (unsigned)m;
-        const bool small = mh == 0;
-        const int z = __clz((int)(small ? ml : mh));
-        const unsigned nh = small ? ml << (z & 31) : __funnelshift_l(ml, mh, z);
-        const unsigned nl = small ? 0u : ml << z;
-        // the top bit, at 63, becomes the significand's implicit one
-        const unsigned lo = __funnelshift_r(nl, nh, 11), r = lo + ((nl >> 10) & 1u);
-        const unsigned e = (unsigned)((1023 + 62 + qc - z - (small ? 32 : 0)) << 20) | ((unsigned)sg & 0x80000000u);
-        const unsigned hi = (nh >> 11) + e + (r < lo ? 1u : 0u);
-        return m == 0 ? 0.0 : __hiloint2double((int)hi, (int)r);
-    }
     // with_fp: the real part by additions
     __device__ __forceinline__ double2 operator()(fxc c, bool with_fp) const
     {
-        double2 o = make_double2(with_fp ? fp(c.x) : integer(c.x), integer(c.y));
+        double2 o = make_double2(with_fp ? fp(c.x) : fx_double(c.x, qc), fx_double(c.y, qc));
         if (bad) o.x = o.y = __longlong_as_double(0x7ff8000000000000LL);
         if (scaled) {
             o.x *= f;

@@ -99,7 +99,7 @@ static int imag_flow(gpss_ctx *c, double dtl, const void *in0, bool pre_nl, void
         const void *ph;
         GPSS_TRY(get_phase(c, axis, dtl, 1, 1, &ph, &a.prow));
         a.phase = (const vec2<T> *)ph;
-        if ((first && pre_nl) || (last && nl_last)) GPSS_TRY(set_nl<T>(c, a, NL_NONE, dtnl));
+        if ((first && pre_nl) || (last && nl_last)) GPSS_TRY(set_nl<T>(c, a, NL_NONE, dtnl, false));
         if (first && pre_nl) {
             a.nl_pre = 1;
             a.scale = c->scale;
@@ -814,7 +814,7 @@ int gpss_time_pass(gpss_ctx *c, int axis, int mode, int reps, double dt, double 
             a.fin_status = c->status;
             CUDA_TRY(c, cudaMemsetAsync(c->status, 0, sizeof(int), c->stream));
         }
-        if (mode == 1) GPSS_TRY(set_nl<T>(c, a, NL_REAL, dt));
+        if (mode == 1) GPSS_TRY(set_nl<T>(c, a, NL_REAL, dt, true));
         GPSS_TRY(launch<T>(c, axis, MODE_FUSED, a));  // warm-up
         CUDA_TRY(c, cudaEventRecord(c->ev[6], c->stream));
         for (int i = 0; i < reps; i++) GPSS_TRY(launch<T>(c, axis, MODE_FUSED, a));

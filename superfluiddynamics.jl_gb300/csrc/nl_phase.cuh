@@ -3,7 +3,9 @@
 //     psi <- exp(-i (V + beta |psi|^2) dt) psi              (real time)
 //     psi <- exp(-(V + beta |psi|^2) dt) psi                 (imaginary time)
 //
-// FP64 fields use the expression as written, in FP64.
+// FP64 fields use the expression as written, in FP64, in the plain form's
+// sweeps; in the passes real time runs on their fixed-point values (fft_fix.cuh)
+// and imaginary time takes its exponential from the integer pipes (NLImag64).
 //
 // FP32 fields: GB300 runs FP64 arithmetic at a small fraction of its FP32
 // rate, so instead of FP64 the phase argument theta = (V + beta|psi|^2) dt is
@@ -192,6 +194,25 @@ __device__ __forceinline__ double2 nl_apply(double2 v, double Vv, const NLConst<
     if (imag) return make_double2(f.x * v.x, f.x * v.y);
     return nl_rotate(f, v);
 }
+
+// The same in imaginary time for the passes of FP64 fields: the exponential on
+// the integer pipes (fx_exp2neg), its argument in units of ln 2 with 1/ln 2 as
+// hi + lo.
+struct NLImag64 {
+    double beta, dh, dl;
+    const long long *tab2;
+    __device__ __forceinline__ NLImag64(double b, double dt, const long long *t) : beta(b), tab2(t)
+    {
+        dh = dt * 1.4426950408889634;
+        dl = fma(dt, 1.4426950408889634, -dh) + dt * 2.0355273740931033e-17;
+    }
+    __device__ __forceinline__ double2 operator()(double2 v, double Vv) const
+    {
+        const double r = fma(beta, v.x * v.x + v.y * v.y, Vv);
+        const double f = fx_exp2neg(fma(r, dh, r * dl), tab2);
+        return make_double2(f * v.x, f * v.y);
+    }
+};
 
 __device__ __forceinline__ float2 nl_factor(float2 v, float Vv, const NLConst<float> &c, bool imag)
 {

@@ -132,7 +132,9 @@ static cudaError_t launch_pass_sized(int mode, const PassArgs<T> &a, int blocks,
         }
         if (!a.phase) return cudaErrorInvalidValue;  // every other fused pass reads a phase table
         // the fixed-point nonlinear flow takes the field unscaled, and its table
-        if (sizeof(T) == 8 && a.nl_mode == NL_REAL && (a.scale || !a.nl_fx.tab)) return cudaErrorInvalidValue;
+        if (sizeof(T) == 8 && a.nl_mode == NL_REAL && a.scale) return cudaErrorInvalidValue;
+        if (sizeof(T) == 8 && (a.nl_mode != NL_NONE || a.nl_pre || a.adj_pre) && !a.nl_fx.tab2)
+            return cudaErrorInvalidValue;
         if (a.nl_pre || a.dot_with) {
             if (diag || acc || adj || a.nl_mode != NL_NONE) return cudaErrorInvalidValue;
             return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_IMAGM | SIZE>(a, blocks, s);

@@ -88,7 +88,7 @@ cudaError_t launch_gen_f64(int mode, const PassArgs<double> &a, const GenPlan &p
 {
     // none of the adjoint, stacked plane or compensated features
     if (a.pre_out || a.adj_pre || a.plane_nl || a.plane_scale || a.comp) return cudaErrorInvalidValue;
-    if (a.nl_mode == NL_REAL && !a.nl_fx.tab) return cudaErrorInvalidValue;
+    if ((a.nl_mode != NL_NONE || a.nl_pre) && !a.nl_fx.tab2) return cudaErrorInvalidValue;
     switch (mode) {
     case MODE_FUSED:
         if (!a.phase && !a.mask_lim) return cudaErrorInvalidValue;

@@ -412,7 +412,7 @@ gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
     const bool scaled = a.scale != nullptr;
     const T scale = scaled ? load_scale<T>(a.scale) : (T)1;
     const bool fxnl = MODE == MODE_FUSED && a.nl_mode == NL_REAL;
-    const bool vbad = fxnl && a.nl_fx.vbad && *a.nl_fx.vbad != 0;
+    const bool vbad = MODE == MODE_FUSED && a.nl_fx.vbad && *a.nl_fx.vbad != 0;
     (void)vbad;
     T acc_mass = 0, acc_pot = 0, acc_int = 0, acc_kin = 0, acc_rot = 0;
     double tot[RQ_COUNT] = {0.0, 0.0, 0.0, 0.0, 0.0};
@@ -439,8 +439,7 @@ gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
             if constexpr (MODE == MODE_FUSED) {
                 if (scaled) x = cscale(x, scale);
                 if (a.nl_pre && valid) {  // chi = N(scale * psi) of the merged imaginary-time step
-                    const NLConst<T> nlc = nl_const<T>(a.nl_split, a.nl_beta, a.nl_dt);
-                    x = nl_apply(x, a.V ? a.V[e] : (T)0, nlc, true);
+                    x = NLImag64(a.nl_beta, a.nl_dt, a.nl_fx.tab2)(x, a.V ? a.V[e] : (T)0);
                     if (a.nl_pre_out) a.nl_pre_out[e] = x;
                 }
             }
@@ -550,7 +549,6 @@ gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
             }
         }
         if constexpr (MODE == MODE_FUSED || MODE == MODE_INV) {
-            const NLConst<T> nlc = nl_const<T>(a.nl_split, a.nl_beta, a.nl_dt);
             int qv = q + (MODE == MODE_FUSED ? p.et + fxpe : p.ei), lsh = 0, rsh = 0;
             if (fxnl) {
                 const int sh = 190 + 2 * qv + a.nl_fx.ge;
@@ -577,7 +575,7 @@ gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
                 if (!valid) continue;
                 if constexpr (MODE == MODE_FUSED) {
                     if (a.nl_mode != NL_NONE && !fxnl) {
-                        v = nl_apply(v, a.V ? a.V[e] : (T)0, nlc, true);  // imaginary time
+                        v = NLImag64(a.nl_beta, a.nl_dt, a.nl_fx.tab2)(v, a.V ? a.V[e] : (T)0);  // imaginary time
                     }
                     if (red & RED_POINT) {
                         const T rho = v.x * v.x + v.y * v.y;

@@ -368,8 +368,9 @@ template <typename T, int N, bool XL, int FEAT = 0> struct PassShape {
     // (FP64 radix-4 stages: the roots of unity in natural order instead)
     static constexpr bool TWB = N1 != N2 && !QUAD;
     // tables: hi and lo (FP32), or one 16-byte fixed-point constant (FP64)
-    // and, where the pass may carry the nonlinear flow, its roots of unity
-    static constexpr int NLTAB = sizeof(T) == 8 && (FEAT & FEAT_NL) != 0 ? FX_NL_TAB : 0;
+    // and, where the pass may carry the nonlinear flow or its adjoint, the flow's
+    // roots of unity (imaginary time: powers of two)
+    static constexpr int NLTAB = sizeof(T) == 8 && (FEAT & (FEAT_NL | FEAT_IMAGM | FEAT_ADJ)) != 0 ? FX_NL_TAB : 0;
     static constexpr int TABLES = (TWB ? 3 : 2) * N * (sizeof(T) == 4 ? 2 : 1) + NLTAB;
     static constexpr int SMEM_SLOTS = STAGE + DATA + TABLES + (TMA ? 2 : 0);
     static constexpr size_t SMEM_BYTES = sizeof(vec2<T>) * SMEM_SLOTS;
@@ -428,7 +429,7 @@ template <typename T, int THREADS>
 __device__ __forceinline__ void finish_reduction(const PassArgs<T> &a, unsigned qmask)
 {
     __shared__ bool last;
-    __shared__ double red[THREADS];
+    __shared__ double fin[RQ_COUNT][THREADS / 32];
     if (threadIdx.x == 0) {
         __threadfence();  // this CTA's partials before its arrival
         const unsigned ticket = atomicAdd(a.counter, 1u);
@@ -437,24 +438,34 @@ __device__ __forceinline__ void finish_reduction(const PassArgs<T> &a, unsigned 
     __syncthreads();
     if (!last) return;
     __threadfence();
-    const int G = gridDim.x;
+    // all quantities side by side, one barrier: the FP64 additions are a chain
+    // of 64 clocks each on this chip, and a small field's pass waits for them
+    // (64^2 solve loop 314 -> 293 us against a tree of barriers per sum)
+    const int G = gridDim.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    double s[RQ_COUNT] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    for (int b = threadIdx.x; b < G; b += THREADS) {
+#pragma unroll
+        for (int q = 0; q < RQ_COUNT; q++)
+            if (qmask & (1u << q)) s[q] += __ldcg(a.partials + (size_t)q * G + b);
+    }
+#pragma unroll
     for (int q = 0; q < RQ_COUNT; q++) {
         if (!(qmask & (1u << q))) continue;
-        double s = 0.0;
-        for (int b = threadIdx.x; b < G; b += THREADS) s += __ldcg(a.partials + (size_t)q * G + b);
-        red[threadIdx.x] = s;
-        __syncthreads();
-#pragma unroll
-        for (int o = THREADS / 2; o > 0; o >>= 1) {
-            if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) a.fin_out[q] = red[0];
-        __syncthreads();
+        for (int o = 16; o > 0; o >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
+        if (lane == 0) fin[q][wid] = s[q];
     }
+    __syncthreads();
+    if (threadIdx.x < RQ_COUNT && (qmask & (1u << threadIdx.x))) {
+        double t = 0.0;
+#pragma unroll
+        for (int i = 0; i < THREADS / 32; i++) t += fin[threadIdx.x][i];
+        a.fin_out[threadIdx.x] = t;
+        if (threadIdx.x == RQ_MASS) fin[RQ_MASS][0] = t;
+    }
+    static_assert(RQ_MASS == 0, "thread 0 has the mass");
     if (threadIdx.x == 0) {
         if (a.fin_mode != FIN_NONE) {
-            const double m = a.fin_out[RQ_MASS];
+            const double m = fin[RQ_MASS][0];
             if (!(m > 0.0) || !isfinite(m)) {
                 *a.fin_status = 1;
                 store_scale(a.fin_scale, 1.0);
@@ -534,10 +545,15 @@ pass_kernel(const PassArgs<T> a)
     // the nonlinear flow in fixed point (FP64, real time)
     const bool fxnl = kFix && kNL && MODE == MODE_FUSED && a.nl_mode == NL_REAL;
     int4 *snl = reinterpret_cast<int4 *>(sph + N);
+    long long *snl2 = reinterpret_cast<long long *>(snl);
     (void)snl;
-    if constexpr (kFix && kNL && MODE == MODE_FUSED) {
-        if (fxnl)
+    (void)snl2;
+    if constexpr (S::NLTAB > 0 && MODE == MODE_FUSED) {
+        if (fxnl || (kAdj && a.adj_pre)) {
             for (int i = tid; i < FX_NL_TAB; i += THREADS) snl[i] = a.nl_fx.tab[i];
+        } else if (a.nl_mode == NL_IMAG || (kImagM && a.nl_pre)) {
+            for (int i = tid; i < FX_NL_TAB; i += THREADS) snl2[i] = a.nl_fx.tab2[i];
+        }
     }
     const int fxpe = kFix && MODE == MODE_FUSED && !kMask ? reinterpret_cast<const int4 *>(a.phase)->x : 0;
     (void)fxpe;
@@ -559,7 +575,7 @@ pass_kernel(const PassArgs<T> a)
     const bool scaled = a.scale != nullptr;
     const T scale = scaled ? load_scale<T>(a.scale) : (T)1;
     const T kmult = a.kmult;
-    const bool vbad = fxnl && a.nl_fx.vbad && *a.nl_fx.vbad != 0;
+    const bool vbad = kFix && MODE == MODE_FUSED && a.nl_fx.vbad && *a.nl_fx.vbad != 0;
     (void)vbad;
     // compensated passes with a mass bound: one grid for every stage (C of
     // the quantum 2^-22 of 32 sqrt(M/2) = 16 sqrt(2 M), rounded up)
@@ -654,13 +670,20 @@ pass_kernel(const PassArgs<T> a)
         }
         if constexpr (MODE == MODE_FUSED && kImagM) {
             if (a.nl_pre) {  // chi = N(scale * psi), kept for the inner product of the last pass
-                const NLConst<T> nlc = nl_const<T>(a.nl_split, a.nl_beta, a.nl_dt);
+                auto prologue = [&](auto flow) {
 #pragma unroll
-                for (int j = 0; j < N1; j++) {
-                    const uint32_t e = base + (uint32_t)(r + N2 * j) * st;
-                    const V u = scaled ? cscale(v[j], scale) : v[j];
-                    v[j] = nl_apply(u, a.V ? a.V[e] : (T)0, nlc, true);
-                    if (valid && a.nl_pre_out) a.nl_pre_out[e] = v[j];
+                    for (int j = 0; j < N1; j++) {
+                        const uint32_t e = base + (uint32_t)(r + N2 * j) * st;
+                        const V u = scaled ? cscale(v[j], scale) : v[j];
+                        v[j] = flow(u, a.V ? a.V[e] : (T)0);
+                        if (valid && a.nl_pre_out) a.nl_pre_out[e] = v[j];
+                    }
+                };
+                if constexpr (kFix) {
+                    prologue(NLImag64(a.nl_beta, a.nl_dt, snl2));
+                } else {
+                    const NLConst<T> nlc = nl_const<T>(a.nl_split, a.nl_beta, a.nl_dt);
+                    prologue([&](V u, T vv) { return nl_apply(u, vv, nlc, true); });
                 }
             }
         }
@@ -1379,19 +1402,36 @@ pass_kernel(const PassArgs<T> a)
                 for (int j = 0; j < N1; j++) a.pre_out[base + (uint32_t)(r + N2 * j) * st] = v[j];
             }
             if (a.adj_pre) {
-                const NLConst<T> nlc = nl_const<T>(a.nl_split, a.nl_beta, a.nl_dt);
-                const T two_beta_dt = (T)(2.0 * a.nl_beta * a.nl_dt);
+                // f: the forward flow's factor at pre (FP64: theta from FP64
+                // |pre|^2, the factor in fixed point, 20 FP64 operations per
+                // cell where FP64 sincos makes it 58: 256^2 adjoint, 200 steps,
+                // 7.45 -> 7.04 ms)
+                auto adjoint = [&](auto factor) {
+                    const T two_beta_dt = (T)(2.0 * a.nl_beta * a.nl_dt);
 #pragma unroll
-                for (int j = 0; j < N1; j++) {
-                    const uint32_t e = base + (uint32_t)(r + N2 * j) * st;
-                    const V pre = a.adj_pre[e];
-                    const T vv = a.V ? a.V[e] : (T)0;
-                    const V f = nl_factor(pre, vv, nlc, false);
-                    const V pout = nl_rotate(f, pre);
-                    const T im = v[j].x * pout.y - v[j].y * pout.x;  // Im(conj(g) psi_out)
-                    if (valid) a.adj_dLdV[e] += a.nl_dt * (double)im;
-                    const V rot = cmulc(v[j], f);                     // conj(f) g
-                    v[j] = mk<V>(rot.x + two_beta_dt * im * pre.x, rot.y + two_beta_dt * im * pre.y);
+                    for (int j = 0; j < N1; j++) {
+                        const uint32_t e = base + (uint32_t)(r + N2 * j) * st;
+                        const V pre = a.adj_pre[e];
+                        const V f = factor(pre, e);
+                        const V pout = nl_rotate(f, pre);
+                        const T im = v[j].x * pout.y - v[j].y * pout.x;  // Im(conj(g) psi_out)
+                        if (valid) a.adj_dLdV[e] += a.nl_dt * (double)im;
+                        const V rot = cmulc(v[j], f);                     // conj(f) g
+                        v[j] = mk<V>(rot.x + two_beta_dt * im * pre.x, rot.y + two_beta_dt * im * pre.y);
+                    }
+                };
+                if constexpr (kFix) {
+                    adjoint([&](V pre, uint32_t e) {
+                        const long long th =
+                            fx_theta(pre.x * pre.x + pre.y * pre.y, a.nl_fx.gh, a.nl_fx.gl, a.nl_fx.ge) +
+                            (a.nl_fx.vturn ? a.nl_fx.vturn[e] : 0);
+                        const fxc f = fx_expi(th, snl);
+                        const double re = fx_double(f.x, -62);
+                        return mk<V>(vbad ? __longlong_as_double(0x7ff8000000000000LL) : re, -fx_double(f.y, -62));
+                    });
+                } else {
+                    const NLConst<T> nlc = nl_const<T>(a.nl_split, a.nl_beta, a.nl_dt);
+                    adjoint([&](V pre, uint32_t e) { return nl_factor(pre, a.V ? a.V[e] : (T)0, nlc, false); });
                 }
             }
         }
@@ -1460,7 +1500,7 @@ pass_kernel(const PassArgs<T> a)
                         if constexpr (sizeof(T) == 4) {
                             v[j] = imag ? nl_apply(v[j], vv, nlc, true) : nl_apply_real_cell(v[j], vv, nlc);
                         } else {
-                            v[j] = nl_apply(v[j], vv, nlc, imag);
+                            v[j] = NLImag64(a.nl_beta, a.nl_dt, snl2)(v[j], vv);  // real time: above
                         }
                     }
                 }

@@ -90,6 +90,7 @@ struct gpss_ctx {
     int *rk_lim = nullptr;    // RK: 2/3-rule limits per inner position (the FEAT_MASK pass)
     void *im_buf = nullptr;   // implicit schemes: work fields (implicit_impl)
     size_t im_bytes = 0;
+    int kry_hint = 0;         // iterations of the last Krylov solve (how many to issue at once)
     // discrete adjoint: buffers kept between calls (sized for adj_nck checkpoints, adj_K states)
     void *adj_buf = nullptr;
     size_t adj_bytes = 0;
@@ -658,7 +659,7 @@ template <typename T> static int nl_plain(gpss_ctx *c, double dt, int imag)
     return GPSS_OK;
 }
 
-// sum |psi|^2 (and V|psi|^2, |psi|^4; with kin also the Parseval sums) of the
+// sum |psi|^2 (with kin also V|psi|^2, |psi|^4 and the Parseval sums) of the
 // current field by read-only passes, into c->sums slot `axis` (kin) or the
 // diagnostics slot (mass only)
 template <typename T> static int diag_passes(gpss_ctx *c, bool kin, int mode)
@@ -666,9 +667,10 @@ template <typename T> static int diag_passes(gpss_ctx *c, bool kin, int mode)
     const int naxes = kin ? c->ndim : 1;
     for (int axis = 0; axis < naxes; axis++) {
         PassArgs<T> a = axis_args<T>(c, axis, c->psi, c->psi);
-        a.red = (axis == 0 ? RED_POINT : 0) | (kin ? RED_KIN : 0);
+        a.red = !kin ? RED_MASS : (axis == 0 ? RED_POINT : 0) | RED_KIN;
         a.V = c->have_V ? (const T *)c->V : nullptr;
-        a.coord = axis == 0 ? c->coord_dev[1] : (axis == 1 ? c->coord_dev[0] : nullptr);
+        if (sizeof(T) == 4 || c->omega != 0.0)  // (FP64 without rotation: no rotation sums)
+            a.coord = axis == 0 ? c->coord_dev[1] : (axis == 1 ? c->coord_dev[0] : nullptr);
         set_finish<T>(c, a, kin ? axis : kDiagSlot, axis == 0 ? mode : FIN_NONE);
         GPSS_TRY(launch<T>(c, axis, MODE_DIAG, a));
     }

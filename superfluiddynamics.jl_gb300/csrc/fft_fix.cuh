@@ -277,6 +277,27 @@ __device__ __forceinline__ fxc fx_expi(long long th, const int4 *tab)
     return f;
 }
 
+// exp(-2 pi i th / 2^64) c / 4, c of modulus at most 2^62
+__device__ __forceinline__ fxc fx_rotate(fxc c, long long th, const int4 *tab)
+{
+    int xh, xl, yh, yl;
+    fx_split(c.x, xh, xl);
+    fx_split(c.y, yh, yl);
+    const fxc f = fx_expi(th, tab);
+    // c conj(f) / 4 (run-time constants are negated whole, not by halves: a
+    // low half of -2^31 has no negative)
+    int fh, fl, gh, gl, nh, nl;
+    fx_split(f.x, fh, fl);
+    fx_split(f.y, gh, gl);
+    fx_split(-f.y, nh, nl);
+    fxc o;
+    o.x = fx_fold(fx_madw(xh, fh, fx_madw(yh, gh, FX_S0)),
+                  fx_madw(xl, fh, fx_madw(yl, gh, fx_madw(xh, fl, fx_madw(yh, gl, FX_X0)))));
+    o.y = fx_fold(fx_madw(yh, fh, fx_madw(xh, nh, FX_S0)),
+                  fx_madw(yl, fh, fx_madw(xl, nh, fx_madw(yh, fl, fx_madw(xh, nl, FX_X0)))));
+    return o;
+}
+
 // One cell: c of modulus at most 2^62; theta = |c|^2 2^-62 (gh 2^32 + gl) 2^-64
 // shifted left by lsh and right by rsh, plus vt.  Returns exp(-i theta) c / 4.
 __device__ __forceinline__ fxc fx_nl_real(fxc c, long long vt, int gh, int gl, int lsh, int rsh, const int4 *tab)
@@ -289,20 +310,7 @@ __device__ __forceinline__ fxc fx_nl_real(fxc c, long long vt, int gh, int gl, i
     const long long S = fx_madw(xh, xh, fx_madw(yh, yh, 0));
     const long long X = fx_madw(xl, xh, fx_madw(yl, yh, kX));
     const long long rho = (S << 2) + (X >> 29);
-    const long long th = ((fx_rmul(rho, gh, gl) << lsh) >> rsh) + vt;
-    const fxc f = fx_expi(th, tab);
-    // c conj(f) / 4 (run-time constants are negated whole, not by halves: a
-    // low half of -2^31 has no negative)
-    int fh, fl, gh2, gl2, nh, nl;
-    fx_split(f.x, fh, fl);
-    fx_split(f.y, gh2, gl2);
-    fx_split(-f.y, nh, nl);
-    fxc o;
-    o.x = fx_fold(fx_madw(xh, fh, fx_madw(yh, gh2, FX_S0)),
-                  fx_madw(xl, fh, fx_madw(yl, gh2, fx_madw(xh, fl, fx_madw(yh, gl2, FX_X0)))));
-    o.y = fx_fold(fx_madw(yh, fh, fx_madw(xh, nh, FX_S0)),
-                  fx_madw(yl, fh, fx_madw(xl, nh, fx_madw(yh, fl, fx_madw(xh, nl, FX_X0)))));
-    return o;
+    return fx_rotate(c, ((fx_rmul(rho, gh, gl) << lsh) >> rsh) + vt, tab);
 }
 
 // theta / (2 pi) of rho = |psi|^2 >= 0 in FP64 (without the potential's part), 2^64

@@ -239,12 +239,6 @@ template <typename T>
 cudaError_t im_rhs_cn(const vec2<T> *phi, const vec2<T> *phi1, const vec2<T> *psim, const vec2<T> *lap, const T *V,
                       double beta, double dt, int tsch, vec2<T> *b, int64_t total, cudaStream_t s);
 template <typename T>
-cudaError_t im_op(const vec2<T> *x, const vec2<T> *lap, int scheme, double dt, const vec2<T> *M, const T *Anl,
-                  const vec2<T> *Anl2, const vec2<T> *b, int precond, vec2<T> *out, int64_t total, cudaStream_t s);
-template <typename T>
-cudaError_t im_dot2(const vec2<T> *a1, const vec2<T> *b1, const vec2<T> *a2, const vec2<T> *b2, int64_t total,
-                    double *partials, double *out, cudaStream_t s);
-template <typename T>
 cudaError_t im_axmy(vec2<T> *out, const vec2<T> *x, double alpha, const vec2<T> *y, int64_t total, cudaStream_t s);
 
 // The scalars of one BiCGStab solve (krylov.jl:1-67), kept on the device so
@@ -259,17 +253,29 @@ struct KrylovDev {
     double normb, rr2, alpha, omega, beta;
     int done, niter, nonfinite, it;
 };
-cudaError_t kry_init(KrylovDev *K, const double *dots, cudaStream_t s);
-cudaError_t kry_alpha(KrylovDev *K, const double *dots, cudaStream_t s);
-cudaError_t kry_omega(KrylovDev *K, const double *dots, cudaStream_t s);
-cudaError_t kry_check(KrylovDev *K, const double *dots, double tol, int nkrylov, cudaStream_t s);
+// what the dot products of a kernel are for (see implicit.cu)
+enum { KRY_NONE = 0, KRY_INIT = 1, KRY_ALPHA = 2, KRY_OMEGA = 3, KRY_CHECK = 4 };
+constexpr int KRY_MAX_CTAS = 304;  // of a kernel with dot products
+struct KryScratch {
+    double *partials;        // [2 * KRY_MAX_CTAS]
+    double *dots;            // the last two sums
+    unsigned int *counter;   // 0 between launches
+    KrylovDev *K;
+};
+template <typename T>
+cudaError_t im_op(const vec2<T> *x, const vec2<T> *lap, int scheme, double dt, const vec2<T> *M, const T *Anl,
+                  const vec2<T> *Anl2, const vec2<T> *b, int precond, vec2<T> *out, int64_t total, const vec2<T> *r,
+                  const vec2<T> *r2, const KryScratch &k, int what, cudaStream_t s);
+template <typename T>
+cudaError_t im_norm2(const vec2<T> *a, int64_t total, const KryScratch &k, int what, cudaStream_t s);
 // s = r - alpha Ap;  phi = (phi + alpha p) + omega s, r = s - omega As;  p = r + beta (p - omega Ap)
 template <typename T>
 cudaError_t im_axmy_k(vec2<T> *out, const vec2<T> *x, const vec2<T> *y, const KrylovDev *K, int64_t total,
                       cudaStream_t s);
 template <typename T>
 cudaError_t im_update_k(vec2<T> *phi, const vec2<T> *p, const vec2<T> *sv, const vec2<T> *As, vec2<T> *r,
-                        const KrylovDev *K, int64_t total, cudaStream_t s);
+                        const vec2<T> *r2, const KryScratch &k, double tol, int nkrylov, int64_t total,
+                        cudaStream_t s);
 template <typename T>
 cudaError_t im_pdir_k(vec2<T> *p, const vec2<T> *r, const vec2<T> *Ap, const KrylovDev *K, int64_t total,
                       cudaStream_t s);

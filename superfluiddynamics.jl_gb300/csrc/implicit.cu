@@ -3,6 +3,7 @@
 // and of their BiCGStab solver (src/NumModels/krylov.jl:1-67).  lapRot comes
 // from the fused directional passes (the host chains them); everything else of
 // a Krylov iteration is here.
+#include <algorithm>
 #include "gpss_internal.h"
 #include "pdl.cuh"
 
@@ -97,16 +98,127 @@ __global__ void k_im_rhs_cn(const vec2<T> *__restrict__ phi, const vec2<T> *__re
     }
 }
 
+// ---- dot products finished in the kernel that has the vectors at hand
+//
+// A BiCGStab iteration needs three pairs of dot products.  They are summed
+// where one of their vectors is formed (the operator's result, the residual):
+// FP64 per thread, per CTA by shuffles, and by the last CTA to arrive over the
+// per-CTA partials in a fixed order; one thread of it then forms the
+// iteration's scalars (KrylovDev).  With kernels of their own for the products,
+// their finish and the scalars an iteration was 19 launches, now 11 (64^3
+// backward Euler, 4 steps, 1696 -> 1590 us).
+struct DotArgs {
+    int what;                // KRY_*
+    double *partials;        // [2][gridDim.x]
+    unsigned int *counter;   // 0 between launches
+    double *out;             // the two sums (nullable)
+    KrylovDev *K;
+    double tol;              // KRY_CHECK
+    int nkrylov;
+};
+
+// the scalars of one solve from two dot products (krylov.jl:1-67, one thread)
+__device__ void kry_scalars(const DotArgs &d, double d0, double d1)
+{
+    KrylovDev *K = d.K;
+    if (d.what == KRY_INIT) {  // normb = sqrt(b.b) (or |M b|), a fresh solve
+        K->normb = sqrt(d0);
+        K->rr2 = K->alpha = K->omega = K->beta = 0.0;
+        K->done = K->niter = K->nonfinite = K->it = 0;
+        return;
+    }
+    if (d.what == KRY_NONE || K->done) return;
+    if (d.what == KRY_ALPHA) {  // iteration it: rr2 = r.r2, alpha = rr2 / (Ap.r2)
+        K->it += 1;
+        K->rr2 = d0;
+        K->alpha = d0 / d1;
+    } else if (d.what == KRY_OMEGA) {  // omega = (As.s) / (As.As)
+        K->omega = d0 / d1;
+    } else {
+        // the stopping test on |r| / normb, then niter = it and beta =
+        // (r.r2) / rr2 * alpha / omega; the last allowed iteration ends the solve
+        if (!isfinite(d0)) {
+            K->nonfinite = 1;
+            K->done = 1;
+        } else if (sqrt(d0) / K->normb < d.tol) {
+            K->done = 1;
+        } else {
+            K->niter = K->it;
+            K->beta = d1 / K->rr2 * K->alpha / K->omega;
+            if (K->it >= d.nkrylov) K->done = 1;
+        }
+    }
+}
+
+// sums of x1 and x2 over the grid (CTAs of 256 threads), then the scalars
+__device__ __forceinline__ void dot_finish(double x1, double x2, const DotArgs &d)
+{
+    __shared__ double s1[8], s2[8];
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    auto cta = [&](double &a, double &b) {  // thread 0 gets the CTA's sums
+        for (int o = 16; o > 0; o >>= 1) {
+            a += __shfl_xor_sync(0xffffffffu, a, o);
+            b += __shfl_xor_sync(0xffffffffu, b, o);
+        }
+        if (lane == 0) {
+            s1[wid] = a;
+            s2[wid] = b;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            a = s1[0];
+            b = s2[0];
+            for (int i = 1; i < 8; i++) {
+                a += s1[i];
+                b += s2[i];
+            }
+        }
+    };
+    cta(x1, x2);
+    if (threadIdx.x == 0) {
+        d.partials[blockIdx.x] = x1;
+        d.partials[gridDim.x + blockIdx.x] = x2;
+        __threadfence();  // the partials before the arrival
+        last = atomicAdd(d.counter, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double a = 0.0, b = 0.0;
+    for (unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x) {
+        a += __ldcg(d.partials + i);
+        b += __ldcg(d.partials + gridDim.x + i);
+    }
+    cta(a, b);
+    if (threadIdx.x == 0) {
+        if (d.out) {
+            d.out[0] = a;
+            d.out[1] = b;
+        }
+        kry_scalars(d, a, b);
+        *d.counter = 0u;
+    }
+}
+
+// Re(a conj b) in FP64
+template <typename T> __device__ __forceinline__ double re_dot(vec2<T> a, vec2<T> b)
+{
+    return (double)a.x * (double)b.x + (double)a.y * (double)b.y;
+}
+
 // out = prodA(x) given lap = lapRot(x) (backward-euler.jl:87-90, 179-189;
 // crank-nicolson.jl:112-114, 234-236, 356-359, 478-481); bsub: out = b - prodA(x);
-// precond: out = M * out
+// precond: out = M * out.  Dots: KRY_ALPHA r.r2 and out.r2; KRY_OMEGA out.x and out.out
 template <typename T>
 __global__ void k_im_op(const vec2<T> *__restrict__ x, const vec2<T> *__restrict__ lap, int scheme, double idt,
                         const vec2<T> *__restrict__ M, const T *__restrict__ Anl, const vec2<T> *__restrict__ Anl2,
-                        const vec2<T> *__restrict__ b, int precond, vec2<T> *__restrict__ out, int64_t total)
+                        const vec2<T> *__restrict__ b, int precond, vec2<T> *__restrict__ out, int64_t total,
+                        const vec2<T> *__restrict__ r, const vec2<T> *__restrict__ r2, const DotArgs d)
 {
     pdl_enter();
     const T id = (T)idt, h = (T)0.5;
+    double x1 = 0.0, x2 = 0.0;
     GRID_LOOP(e, total) {
         const vec2<T> v = x[e], L = lap[e];
         T ox, oy;
@@ -158,69 +270,30 @@ __global__ void k_im_op(const vec2<T> *__restrict__ x, const vec2<T> *__restrict
             const T tx = m.x * ox - m.y * oy, ty = m.x * oy + m.y * ox;
             ox = tx; oy = ty;
         }
-        out[e] = mk<vec2<T>>(ox, oy);
+        const vec2<T> o = mk<vec2<T>>(ox, oy);
+        out[e] = o;
+        if (d.what == KRY_ALPHA) {
+            const vec2<T> w = r2[e];
+            x1 += re_dot<T>(r[e], w);
+            x2 += re_dot<T>(o, w);
+        } else if (d.what == KRY_OMEGA) {
+            x1 += re_dot<T>(o, v);
+            x2 += re_dot<T>(o, o);
+        }
     }
+    if (d.what != KRY_NONE) dot_finish(x1, x2, d);
 }
 
 // ---- BiCGStab vector operations (krylov.jl)
 
-// partials[2 * block + {0, 1}] = per-CTA sums of Re(a1 conj b1), Re(a2 conj b2) in FP64
+// a.a, its sum to d.out or into the scalars
 template <typename T>
-__global__ void k_im_dot2(const vec2<T> *__restrict__ a1, const vec2<T> *__restrict__ b1,
-                          const vec2<T> *__restrict__ a2, const vec2<T> *__restrict__ b2, int64_t total,
-                          double *__restrict__ partials)
+__global__ void k_im_norm2(const vec2<T> *__restrict__ a, int64_t total, const DotArgs d)
 {
     pdl_enter();
-    __shared__ double s1[256], s2[256];
-    double x1 = 0.0, x2 = 0.0;
-    GRID_LOOP(e, total) {
-        const vec2<T> p = a1[e], q = b1[e];
-        x1 += (double)p.x * (double)q.x + (double)p.y * (double)q.y;
-        if (a2) {
-            const vec2<T> u = a2[e], w = b2[e];
-            x2 += (double)u.x * (double)w.x + (double)u.y * (double)w.y;
-        }
-    }
-    s1[threadIdx.x] = x1;
-    s2[threadIdx.x] = x2;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) {
-            s1[threadIdx.x] += s1[threadIdx.x + o];
-            s2[threadIdx.x] += s2[threadIdx.x + o];
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        partials[2 * blockIdx.x] = s1[0];
-        partials[2 * blockIdx.x + 1] = s2[0];
-    }
-}
-
-// out[0..1] = the sums of the partials (fixed order), one CTA
-__global__ void k_im_dot_finish(const double *__restrict__ partials, int nblocks, double *__restrict__ out)
-{
-    pdl_enter();
-    __shared__ double s1[256], s2[256];
-    double x1 = 0.0, x2 = 0.0;
-    for (int i = threadIdx.x; i < nblocks; i += blockDim.x) {
-        x1 += partials[2 * i];
-        x2 += partials[2 * i + 1];
-    }
-    s1[threadIdx.x] = x1;
-    s2[threadIdx.x] = x2;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) {
-            s1[threadIdx.x] += s1[threadIdx.x + o];
-            s2[threadIdx.x] += s2[threadIdx.x + o];
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        out[0] = s1[0];
-        out[1] = s2[0];
-    }
+    double x = 0.0;
+    GRID_LOOP(e, total) { x += re_dot<T>(a[e], a[e]); }
+    dot_finish(x, 0.0, d);
 }
 
 // out = x - alpha y
@@ -234,53 +307,6 @@ __global__ void k_im_axmy(vec2<T> *__restrict__ out, const vec2<T> *__restrict__
         const vec2<T> u = x[e], w = y[e];
         out[e] = mk<vec2<T>>(u.x - a * w.x, u.y - a * w.y);
     }
-}
-
-// ---- the solve's scalars on the device (one thread each; KrylovDev)
-
-// normb = sqrt(b.b) (or |M b|), a fresh solve
-__global__ void k_kry_init(KrylovDev *K, const double *__restrict__ dots)
-{
-    pdl_enter();
-    K->normb = sqrt(dots[0]);
-    K->rr2 = K->alpha = K->omega = K->beta = 0.0;
-    K->done = K->niter = K->nonfinite = K->it = 0;
-}
-// iteration it: rr2 = r.r2, alpha = rr2 / (Ap.r2)
-__global__ void k_kry_alpha(KrylovDev *K, const double *__restrict__ dots)
-{
-    pdl_enter();
-    if (K->done) return;
-    K->it += 1;
-    K->rr2 = dots[0];
-    K->alpha = dots[0] / dots[1];
-}
-// omega = (As.s) / (As.As)
-__global__ void k_kry_omega(KrylovDev *K, const double *__restrict__ dots)
-{
-    pdl_enter();
-    if (K->done) return;
-    K->omega = dots[0] / dots[1];
-}
-// the stopping test on |r| / normb, then niter = it and beta = (r.r2) / rr2 *
-// alpha / omega; the last allowed iteration ends the solve
-__global__ void k_kry_check(KrylovDev *K, const double *__restrict__ dots, double tol, int nkrylov)
-{
-    pdl_enter();
-    if (K->done) return;
-    const double rr = dots[0];
-    if (!isfinite(rr)) {
-        K->nonfinite = 1;
-        K->done = 1;
-        return;
-    }
-    if (sqrt(rr) / K->normb < tol) {
-        K->done = 1;
-        return;
-    }
-    K->niter = K->it;
-    K->beta = dots[1] / K->rr2 * K->alpha / K->omega;
-    if (K->it >= nkrylov) K->done = 1;
 }
 
 // s = r - alpha Ap (alpha from the device)
@@ -297,20 +323,25 @@ __global__ void k_im_axmy_k(vec2<T> *__restrict__ out, const vec2<T> *__restrict
     }
 }
 
-// phi = (phi + alpha p) + omega s;  r = s - omega As
+// phi = (phi + alpha p) + omega s;  r = s - omega As;  KRY_CHECK on r.r and r.r2
 template <typename T>
 __global__ void k_im_update_k(vec2<T> *__restrict__ phi, const vec2<T> *__restrict__ p,
                               const vec2<T> *__restrict__ s, const vec2<T> *__restrict__ As, vec2<T> *__restrict__ r,
-                              const KrylovDev *__restrict__ K, int64_t total)
+                              const vec2<T> *__restrict__ r2, const KrylovDev *K, int64_t total, const DotArgs d)
 {
     pdl_enter();
-    if (K->done) return;
+    if (K->done) return;  // (the last CTA, which may set it, arrives after every CTA has read it)
     const T a = (T)K->alpha, w = (T)K->omega;
+    double x1 = 0.0, x2 = 0.0;
     GRID_LOOP(e, total) {
         const vec2<T> f = phi[e], pp = p[e], ss = s[e], aa = As[e];
         phi[e] = mk<vec2<T>>((f.x + a * pp.x) + w * ss.x, (f.y + a * pp.y) + w * ss.y);
-        r[e] = mk<vec2<T>>(ss.x - w * aa.x, ss.y - w * aa.y);
+        const vec2<T> rr = mk<vec2<T>>(ss.x - w * aa.x, ss.y - w * aa.y);
+        r[e] = rr;
+        x1 += re_dot<T>(rr, rr);
+        x2 += re_dot<T>(rr, r2[e]);
     }
+    dot_finish(x1, x2, d);
 }
 
 // p = r + beta (p - omega Ap)
@@ -341,6 +372,23 @@ __global__ void k_im_mfield(vec2<T> *__restrict__ out, const vec2<T> *__restrict
 }
 
 // ---- host launchers
+
+// Kernels that end in dot_finish: four cells per thread, at most two CTAs per
+// SM, so that the FP64 sums across a CTA (a chain of 64 clocks each) are few
+// beside the cells' own.
+static int dot_grid(int64_t total) { return (int)std::min<int64_t>((total + 1023) / 1024, KRY_MAX_CTAS); }
+static DotArgs dot_args(const KryScratch &k, int what)
+{
+    DotArgs d;
+    d.what = what;
+    d.partials = k.partials;
+    d.counter = k.counter;
+    d.out = k.dots;
+    d.K = k.K;
+    d.tol = 0.0;
+    d.nkrylov = 0;
+    return d;
+}
 
 template <typename T>
 cudaError_t im_mfield(vec2<T> *out, const vec2<T> *M, const vec2<T> *x, int64_t total, cudaStream_t s)
@@ -378,22 +426,18 @@ cudaError_t im_rhs_cn(const vec2<T> *phi, const vec2<T> *phi1, const vec2<T> *ps
 
 template <typename T>
 cudaError_t im_op(const vec2<T> *x, const vec2<T> *lap, int scheme, double dt, const vec2<T> *M, const T *Anl,
-                  const vec2<T> *Anl2, const vec2<T> *b, int precond, vec2<T> *out, int64_t total, cudaStream_t s)
+                  const vec2<T> *Anl2, const vec2<T> *b, int precond, vec2<T> *out, int64_t total, const vec2<T> *r,
+                  const vec2<T> *r2, const KryScratch &k, int what, cudaStream_t s)
 {
-    launch_pdl(k_im_op<T>, dim3(im_grid(total)), dim3(256), 0, s,
-               x, lap, scheme, 1.0 / dt, M, Anl, Anl2, b, precond, out, total);
+    launch_pdl(k_im_op<T>, dim3(what == KRY_NONE ? im_grid(total) : dot_grid(total)), dim3(256), 0, s,
+               x, lap, scheme, 1.0 / dt, M, Anl, Anl2, b, precond, out, total, r, r2, dot_args(k, what));
     return cudaGetLastError();
 }
 
 template <typename T>
-cudaError_t im_dot2(const vec2<T> *a1, const vec2<T> *b1, const vec2<T> *a2, const vec2<T> *b2, int64_t total,
-                    double *partials, double *out, cudaStream_t s)
+cudaError_t im_norm2(const vec2<T> *a, int64_t total, const KryScratch &k, int what, cudaStream_t s)
 {
-    const int g = im_grid(total);
-    launch_pdl(k_im_dot2<T>, dim3(g), dim3(256), 0, s, a1, b1, a2, b2, total, partials);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    launch_pdl(k_im_dot_finish, dim3(1), dim3(256), 0, s, partials, g, out);
+    launch_pdl(k_im_norm2<T>, dim3(dot_grid(total)), dim3(256), 0, s, a, total, dot_args(k, what));
     return cudaGetLastError();
 }
 
@@ -401,27 +445,6 @@ template <typename T>
 cudaError_t im_axmy(vec2<T> *out, const vec2<T> *x, double alpha, const vec2<T> *y, int64_t total, cudaStream_t s)
 {
     launch_pdl(k_im_axmy<T>, dim3(im_grid(total)), dim3(256), 0, s, out, x, alpha, y, total);
-    return cudaGetLastError();
-}
-
-cudaError_t kry_init(KrylovDev *K, const double *dots, cudaStream_t s)
-{
-    launch_pdl(k_kry_init, dim3(1), dim3(1), 0, s, K, dots);
-    return cudaGetLastError();
-}
-cudaError_t kry_alpha(KrylovDev *K, const double *dots, cudaStream_t s)
-{
-    launch_pdl(k_kry_alpha, dim3(1), dim3(1), 0, s, K, dots);
-    return cudaGetLastError();
-}
-cudaError_t kry_omega(KrylovDev *K, const double *dots, cudaStream_t s)
-{
-    launch_pdl(k_kry_omega, dim3(1), dim3(1), 0, s, K, dots);
-    return cudaGetLastError();
-}
-cudaError_t kry_check(KrylovDev *K, const double *dots, double tol, int nkrylov, cudaStream_t s)
-{
-    launch_pdl(k_kry_check, dim3(1), dim3(1), 0, s, K, dots, tol, nkrylov);
     return cudaGetLastError();
 }
 
@@ -435,9 +458,14 @@ cudaError_t im_axmy_k(vec2<T> *out, const vec2<T> *x, const vec2<T> *y, const Kr
 
 template <typename T>
 cudaError_t im_update_k(vec2<T> *phi, const vec2<T> *p, const vec2<T> *sv, const vec2<T> *As, vec2<T> *r,
-                        const KrylovDev *K, int64_t total, cudaStream_t s)
+                        const vec2<T> *r2, const KryScratch &k, double tol, int nkrylov, int64_t total,
+                        cudaStream_t s)
 {
-    launch_pdl(k_im_update_k<T>, dim3(im_grid(total)), dim3(256), 0, s, phi, p, sv, As, r, K, total);
+    DotArgs d = dot_args(k, KRY_CHECK);
+    d.tol = tol;
+    d.nkrylov = nkrylov;
+    launch_pdl(k_im_update_k<T>, dim3(dot_grid(total)), dim3(256), 0, s, phi, p, sv, As, r, r2,
+               (const KrylovDev *)k.K, total, d);
     return cudaGetLastError();
 }
 
@@ -457,14 +485,14 @@ cudaError_t im_pdir_k(vec2<T> *p, const vec2<T> *r, const vec2<T> *Ap, const Kry
     template cudaError_t im_rhs_cn<T>(const vec2<T> *, const vec2<T> *, const vec2<T> *, const vec2<T> *,           \
                                       const T *, double, double, int, vec2<T> *, int64_t, cudaStream_t);            \
     template cudaError_t im_op<T>(const vec2<T> *, const vec2<T> *, int, double, const vec2<T> *, const T *,        \
-                                  const vec2<T> *, const vec2<T> *, int, vec2<T> *, int64_t, cudaStream_t);        \
-    template cudaError_t im_dot2<T>(const vec2<T> *, const vec2<T> *, const vec2<T> *, const vec2<T> *, int64_t,    \
-                                    double *, double *, cudaStream_t);                                              \
+                                  const vec2<T> *, const vec2<T> *, int, vec2<T> *, int64_t, const vec2<T> *,       \
+                                  const vec2<T> *, const KryScratch &, int, cudaStream_t);                          \
+    template cudaError_t im_norm2<T>(const vec2<T> *, int64_t, const KryScratch &, int, cudaStream_t);              \
     template cudaError_t im_axmy<T>(vec2<T> *, const vec2<T> *, double, const vec2<T> *, int64_t, cudaStream_t);    \
     template cudaError_t im_axmy_k<T>(vec2<T> *, const vec2<T> *, const vec2<T> *, const KrylovDev *, int64_t,      \
                                       cudaStream_t);                                                                \
     template cudaError_t im_update_k<T>(vec2<T> *, const vec2<T> *, const vec2<T> *, const vec2<T> *, vec2<T> *,    \
-                                        const KrylovDev *, int64_t, cudaStream_t);                                  \
+                                        const vec2<T> *, const KryScratch &, double, int, int64_t, cudaStream_t);   \
     template cudaError_t im_pdir_k<T>(vec2<T> *, const vec2<T> *, const vec2<T> *, const KrylovDev *, int64_t,      \
                                       cudaStream_t);                                                                \
     template cudaError_t im_mfield<T>(vec2<T> *, const vec2<T> *, const vec2<T> *, int64_t, cudaStream_t);

@@ -437,18 +437,21 @@ gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
             const uint32_t e = base + (uint32_t)i * st;
             V x = valid ? a.in[e] : mk<V>((T)0, (T)0);
             if constexpr (MODE == MODE_FUSED) {
-                if (scaled) x = cscale(x, scale);
-                if (a.nl_pre && valid) {  // chi = N(scale * psi) of the merged imaginary-time step
-                    x = NLImag64(a.nl_beta, a.nl_dt, a.nl_fx.tab2)(x, a.V ? a.V[e] : (T)0);
-                    if (a.nl_pre_out) a.nl_pre_out[e] = x;
+                if (a.nl_pre) {  // chi = N(scale * psi) of the merged imaginary-time step
+                    x = NLImag64(a.nl_beta, a.nl_dt, scale, a.nl_fx.tab2)(x, a.V && valid ? a.V[e] : (T)0);
+                    if (a.nl_pre_out && valid) a.nl_pre_out[e] = x;
+                } else if (scaled) {
+                    x = cscale(x, scale);
                 }
             }
             if constexpr (MODE == MODE_DIAG) {
-                if ((red & RED_POINT) && valid) {
+                if ((red & (RED_POINT | RED_MASS)) && valid) {
                     const T rho = x.x * x.x + x.y * x.y;
                     acc_mass += rho;
-                    acc_int += rho * rho;
-                    if (a.V) acc_pot += a.V[e] * rho;
+                    if (red & RED_POINT) {
+                        acc_int += rho * rho;
+                        if (a.V) acc_pot += a.V[e] * rho;
+                    }
                 }
             }
             const int slot = at(MODE == MODE_INV ? pos_of[i] : i);
@@ -457,6 +460,13 @@ gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
             const float hy = fabsf(__int_as_float(__double2hiint(x.y)));
             asm("max.NaN.f32 %0, %0, %1;" : "+f"(top) : "f"(hx));
             asm("max.NaN.f32 %0, %0, %1;" : "+f"(top) : "f"(hy));
+        }
+        if (MODE == MODE_DIAG && !(red & RED_KIN)) {  // no spectrum wanted
+            tot[RQ_MASS] += (double)acc_mass;
+            tot[RQ_POT] += (double)acc_pot;
+            tot[RQ_INT] += (double)acc_int;
+            acc_mass = acc_pot = acc_int = (T)0;
+            continue;
         }
         // ---- the line's quantum from its 2-norm (sums of squares in whole units
         // of 2^-16, so that their order does not matter)
@@ -575,7 +585,7 @@ gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
                 if (!valid) continue;
                 if constexpr (MODE == MODE_FUSED) {
                     if (a.nl_mode != NL_NONE && !fxnl) {
-                        v = NLImag64(a.nl_beta, a.nl_dt, a.nl_fx.tab2)(v, a.V ? a.V[e] : (T)0);  // imaginary time
+                        v = NLImag64(a.nl_beta, a.nl_dt, 1.0, a.nl_fx.tab2)(v, a.V ? a.V[e] : (T)0);  // imaginary time
                     }
                     if (red & RED_POINT) {
                         const T rho = v.x * v.x + v.y * v.y;

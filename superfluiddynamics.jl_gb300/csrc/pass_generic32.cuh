@@ -248,15 +248,24 @@ gen32_tile_kernel(const PassArgs<float> a, const Gen32Plan p)
                 const int64_t e = gbase(g) + (int64_t)pos * a.stride;
                 x = a.in[e];
                 if constexpr (MODE == MODE_DIAG) {
-                    if (red & RED_POINT) {
+                    if (red & (RED_POINT | RED_MASS)) {
                         const T rho = x.x * x.x + x.y * x.y;
                         acc_mass += rho;
-                        acc_int += rho * rho;
-                        if (a.V) acc_pot += a.V[e] * rho;
+                        if (red & RED_POINT) {
+                            acc_int += rho * rho;
+                            if (a.V) acc_pot += a.V[e] * rho;
+                        }
                     }
                 }
             }
             buf0[pos * W + w] = x;
+        }
+        if (MODE == MODE_DIAG && !(red & RED_KIN)) {  // no spectrum wanted
+            tot[RQ_MASS] += (double)acc_mass;
+            tot[RQ_POT] += (double)acc_pot;
+            tot[RQ_INT] += (double)acc_int;
+            acc_mass = acc_pot = acc_int = (T)0;
+            continue;
         }
         __syncthreads();
         V *spec = gen32_tile_fft<-1>(buf0, buf1, p, roots);  // X[k] at k * W + w

@@ -674,16 +674,15 @@ pass_kernel(const PassArgs<T> a)
 #pragma unroll
                     for (int j = 0; j < N1; j++) {
                         const uint32_t e = base + (uint32_t)(r + N2 * j) * st;
-                        const V u = scaled ? cscale(v[j], scale) : v[j];
-                        v[j] = flow(u, a.V ? a.V[e] : (T)0);
+                        v[j] = flow(v[j], a.V ? a.V[e] : (T)0);
                         if (valid && a.nl_pre_out) a.nl_pre_out[e] = v[j];
                     }
                 };
                 if constexpr (kFix) {
-                    prologue(NLImag64(a.nl_beta, a.nl_dt, snl2));
+                    prologue(NLImag64(a.nl_beta, a.nl_dt, (double)scale, snl2));
                 } else {
                     const NLConst<T> nlc = nl_const<T>(a.nl_split, a.nl_beta, a.nl_dt);
-                    prologue([&](V u, T vv) { return nl_apply(u, vv, nlc, true); });
+                    prologue([&](V u, T vv) { return nl_apply(scaled ? cscale(u, scale) : u, vv, nlc, true); });
                 }
             }
         }
@@ -696,6 +695,19 @@ pass_kernel(const PassArgs<T> a)
                     acc_int += rho * rho;
                     if (a.V) acc_pot += a.V[base + (uint32_t)(r + N2 * j) * st] * rho;
                 }
+            } else if (red & RED_MASS) {
+#pragma unroll
+                for (int j = 0; j < N1; j++) {
+                    T rho = v[j].x * v[j].x + v[j].y * v[j].y;
+                    acc_mass += rho;
+                }
+            }
+            if (!(red & RED_KIN)) {  // no spectrum wanted: the transform is left out
+                tot[RQ_MASS] += (double)acc_mass;
+                tot[RQ_POT] += (double)acc_pot;
+                tot[RQ_INT] += (double)acc_int;
+                acc_mass = acc_pot = acc_int = (T)0;
+                continue;
             }
         }
         if constexpr (!kComp && !kFix) dft<N1, -1>(v);
@@ -787,18 +799,17 @@ pass_kernel(const PassArgs<T> a)
             c[j].x = fx_from(v[j].x, 1084 + q);
             c[j].y = fx_from(v[j].y, 1084 + q);
         }
-        // Parseval sums of the values X[k] of this thread (of quantum 2^qs)
+        // Parseval sums of the values X[k] of this thread, in units of kmult^2 and kmult
         auto kin = [&](const fxc &u, int k, const FxOut &os, T &s2, T &s1) {
             const int kk = k < N / 2 ? k : k - N;
-            const T xi = (T)kk * kmult;
             const V X = os(u, false);
             const T m2 = X.x * X.x + X.y * X.y;
-            s2 += xi * xi * m2;
-            s1 += xi * m2;
+            s2 += (T)(kk * kk) * m2;
+            if (a.coord) s1 += (T)kk * m2;
         };
         auto kin_add = [&](T s2, T s1) {
-            acc_kin += s2 * (T)(1.0 / N);
-            if (a.coord) acc_rot += s1 * (T)(1.0 / N) * (T)a.coord[row];
+            acc_kin += s2 * (kmult * kmult * (T)(1.0 / N));
+            if (a.coord) acc_rot += s1 * (kmult * (T)(1.0 / N)) * (T)a.coord[row];
         };
         (void)kin;
         (void)kin_add;
@@ -1097,6 +1108,23 @@ pass_kernel(const PassArgs<T> a)
                         c[j] = fx_nl_real(c[j], vt, a.nl_fx.gh, a.nl_fx.gl, lsh, rsh, snl);
                     }
                     qv += 2;
+                }
+            }
+            // the adjoint of the flow at the state pre: here its rotation, g <-
+            // exp(i theta) g; the rest in the epilogue
+            if constexpr (MODE == MODE_FUSED && kAdj) {
+                if (a.adj_pre) {
+                    constexpr int KS = kQuad ? (kOdd ? 1 : 0) : 2 - (FxLog<N>::V - (N2 > 1 ? 6 : 2));
+                    qv += 2 - KS;
+#pragma unroll
+                    for (int j = 0; j < N1; j++) {
+                        const uint32_t e = base + (uint32_t)(r + N2 * j) * st;
+                        const V pre = a.adj_pre[e];
+                        const long long th =
+                            fx_theta(pre.x * pre.x + pre.y * pre.y, a.nl_fx.gh, a.nl_fx.gl, a.nl_fx.ge) +
+                            (a.nl_fx.vturn ? a.nl_fx.vturn[e] : 0);
+                        c[j] = fx_rotate(fxc{c[j].x << KS, c[j].y << KS}, -th, snl);
+                    }
                 }
             }
             const FxOut oc(qv, bad || vbad, (double)tscale, MODE == MODE_FUSED && tscaled);
@@ -1402,36 +1430,29 @@ pass_kernel(const PassArgs<T> a)
                 for (int j = 0; j < N1; j++) a.pre_out[base + (uint32_t)(r + N2 * j) * st] = v[j];
             }
             if (a.adj_pre) {
-                // f: the forward flow's factor at pre (FP64: theta from FP64
-                // |pre|^2, the factor in fixed point, 20 FP64 operations per
-                // cell where FP64 sincos makes it 58: 256^2 adjoint, 200 steps,
-                // 7.45 -> 7.04 ms)
-                auto adjoint = [&](auto factor) {
-                    const T two_beta_dt = (T)(2.0 * a.nl_beta * a.nl_dt);
+                const NLConst<T> nlc = nl_const<T>(a.nl_split, a.nl_beta, a.nl_dt);
+                const T two_beta_dt = (T)(2.0 * a.nl_beta * a.nl_dt);
 #pragma unroll
-                    for (int j = 0; j < N1; j++) {
-                        const uint32_t e = base + (uint32_t)(r + N2 * j) * st;
-                        const V pre = a.adj_pre[e];
-                        const V f = factor(pre, e);
+                for (int j = 0; j < N1; j++) {
+                    const uint32_t e = base + (uint32_t)(r + N2 * j) * st;
+                    const V pre = a.adj_pre[e];
+                    if constexpr (kFix) {
+                        // v = conj(f) g already, and Im(conj(g) f pre) =
+                        // Im(conj(conj(f) g) pre): 8 FP64 operations per cell, where
+                        // sincos and two FP64 rotations made it 58 (256^2
+                        // adjoint, 200 steps, 7.45 -> 6.8 ms)
+                        const T im = v[j].x * pre.y - v[j].y * pre.x;
+                        if (valid) a.adj_dLdV[e] += a.nl_dt * (double)im;
+                        v[j] = mk<V>(v[j].x + two_beta_dt * im * pre.x, v[j].y + two_beta_dt * im * pre.y);
+                    } else {
+                        const T vv = a.V ? a.V[e] : (T)0;
+                        const V f = nl_factor(pre, vv, nlc, false);
                         const V pout = nl_rotate(f, pre);
                         const T im = v[j].x * pout.y - v[j].y * pout.x;  // Im(conj(g) psi_out)
                         if (valid) a.adj_dLdV[e] += a.nl_dt * (double)im;
                         const V rot = cmulc(v[j], f);                     // conj(f) g
                         v[j] = mk<V>(rot.x + two_beta_dt * im * pre.x, rot.y + two_beta_dt * im * pre.y);
                     }
-                };
-                if constexpr (kFix) {
-                    adjoint([&](V pre, uint32_t e) {
-                        const long long th =
-                            fx_theta(pre.x * pre.x + pre.y * pre.y, a.nl_fx.gh, a.nl_fx.gl, a.nl_fx.ge) +
-                            (a.nl_fx.vturn ? a.nl_fx.vturn[e] : 0);
-                        const fxc f = fx_expi(th, snl);
-                        const double re = fx_double(f.x, -62);
-                        return mk<V>(vbad ? __longlong_as_double(0x7ff8000000000000LL) : re, -fx_double(f.y, -62));
-                    });
-                } else {
-                    const NLConst<T> nlc = nl_const<T>(a.nl_split, a.nl_beta, a.nl_dt);
-                    adjoint([&](V pre, uint32_t e) { return nl_factor(pre, a.V ? a.V[e] : (T)0, nlc, false); });
                 }
             }
         }
@@ -1500,7 +1521,7 @@ pass_kernel(const PassArgs<T> a)
                         if constexpr (sizeof(T) == 4) {
                             v[j] = imag ? nl_apply(v[j], vv, nlc, true) : nl_apply_real_cell(v[j], vv, nlc);
                         } else {
-                            v[j] = NLImag64(a.nl_beta, a.nl_dt, snl2)(v[j], vv);  // real time: above
+                            v[j] = NLImag64(a.nl_beta, a.nl_dt, 1.0, snl2)(v[j], vv);  // real time: above
                         }
                     }
                 }
@@ -1514,7 +1535,16 @@ pass_kernel(const PassArgs<T> a)
                     if (a.V) acc_pot += a.V[base + (uint32_t)(r + N2 * j) * st] * rho;
                 }
             } else if (red & RED_MASS) {
-                if (kImagM && a.dot_with) {
+                if (kFix) {  // four chains: an FP64 addition takes 64 clocks of one warp here
+                    T m[4] = {0, 0, 0, 0};
+#pragma unroll
+                    for (int j = 0; j < N1; j++) {
+                        V w = v[j];
+                        if (kImagM && a.dot_with) w = a.dot_with[base + (uint32_t)(r + N2 * j) * st];
+                        m[j & 3] += w.x * v[j].x + w.y * v[j].y;
+                    }
+                    acc_mass += (m[0] + m[1]) + (m[2] + m[3]);
+                } else if (kImagM && a.dot_with) {
 #pragma unroll
                     for (int j = 0; j < N1; j++) {
                         const V w = a.dot_with[base + (uint32_t)(r + N2 * j) * st];

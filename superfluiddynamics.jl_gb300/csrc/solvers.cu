@@ -151,28 +151,31 @@ template <typename T> static int rk_step_impl(gpss_ctx *c, int nsteps, int stepp
 
 struct ImBufs {
     void *r, *r2, *p, *Ap, *s, *As, *lap, *b, *M, *Anl2, *psim, *phi1, *phiw, *Anl;
-    double *partials, *dots;
-    KrylovDev *kry;
+    KryScratch k;
 };
 
 template <typename T> static int im_bufs(gpss_ctx *c, ImBufs &B)
 {
-    const size_t fb = (size_t)c->total * sizeof(vec2<T>);
-    const size_t rb = (size_t)c->total * sizeof(T);
-    const size_t pb = sizeof(double) * (2 * 152 * 8 + 2) + sizeof(KrylovDev);
+    const size_t fb = ((size_t)c->total * sizeof(vec2<T>) + 15) / 16 * 16;
+    const size_t rb = ((size_t)c->total * sizeof(T) + 15) / 16 * 16;  // what follows is aligned
+    const size_t pb = sizeof(double) * (2 * KRY_MAX_CTAS + 2) + sizeof(KrylovDev) + 16;
     const size_t need = 13 * fb + rb + pb;
+    bool fresh = false;
     if (!c->im_buf || c->im_bytes < need) {
         if (c->im_buf) { cudaStreamSynchronize(c->stream); cudaFree(c->im_buf); c->im_buf = nullptr; }
         GPSS_TRY(dev_alloc(c, &c->im_buf, need));
         c->im_bytes = need;
+        fresh = true;
     }
     char *base = static_cast<char *>(c->im_buf);
     void **f[13] = {&B.r, &B.r2, &B.p, &B.Ap, &B.s, &B.As, &B.lap, &B.b, &B.M, &B.Anl2, &B.psim, &B.phi1, &B.phiw};
     for (int i = 0; i < 13; i++) *f[i] = base + (size_t)i * fb;
     B.Anl = base + 13 * fb;
-    B.partials = reinterpret_cast<double *>(base + 13 * fb + rb);
-    B.dots = B.partials + 2 * 152 * 8;
-    B.kry = reinterpret_cast<KrylovDev *>(B.dots + 2);
+    B.k.partials = reinterpret_cast<double *>(base + 13 * fb + rb);
+    B.k.dots = B.k.partials + 2 * KRY_MAX_CTAS;
+    B.k.K = reinterpret_cast<KrylovDev *>(B.k.dots + 2);
+    B.k.counter = reinterpret_cast<unsigned int *>(B.k.K + 1);
+    if (fresh) CUDA_TRY(c, cudaMemsetAsync(B.k.counter, 0, sizeof(unsigned int), c->stream));
     return GPSS_OK;
 }
 
@@ -183,36 +186,37 @@ template <typename T> static int im_bufs(gpss_ctx *c, ImBufs &B)
         c->launches++;                                                                 \
     } while (0)
 
-// two dot products Sum Re(a conj b) (FP64) read back to the host
-template <typename T>
-static int im_dots(gpss_ctx *c, ImBufs &B, const void *a1, const void *b1, const void *a2, const void *b2,
-                   double out[2])
+// Sum |a|^2 (FP64) read back to the host
+template <typename T> static int im_norm2_host(gpss_ctx *c, ImBufs &B, const void *a, double *out)
 {
     using V = vec2<T>;
-    IM_TRY(im_dot2<T>((const V *)a1, (const V *)b1, (const V *)a2, (const V *)b2, c->total, B.partials, B.dots,
-                      c->stream));
-    CUDA_TRY(c, cudaMemcpyAsync(out, B.dots, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    IM_TRY(im_norm2<T>((const V *)a, c->total, B.k, KRY_NONE, c->stream));
+    CUDA_TRY(c, cudaMemcpyAsync(out, B.k.dots, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));
     return GPSS_OK;
 }
 
-// out = [M] prodA(x) or [M](b - prodA(x))
+// out = [M] prodA(x) or [M](b - prodA(x)), with the dot products of KRY_ALPHA or
+// KRY_OMEGA on the way
 template <typename T>
-static int im_apply(gpss_ctx *c, ImBufs &B, int scheme, double dt, const void *x, bool bsub, int precond, void *out)
+static int im_apply(gpss_ctx *c, ImBufs &B, int scheme, double dt, const void *x, bool bsub, int precond, void *out,
+                    int what = KRY_NONE)
 {
     using V = vec2<T>;
     GPSS_TRY(lap_rot_dev<T>(c, x, B.lap));
     IM_TRY(im_op<T>((const V *)x, (const V *)B.lap, scheme, dt, (const V *)B.M, (const T *)B.Anl,
-                    (const V *)B.Anl2, bsub ? (const V *)B.b : nullptr, precond, (V *)out, c->total, c->stream));
+                    (const V *)B.Anl2, bsub ? (const V *)B.b : nullptr, precond, (V *)out, c->total,
+                    (const V *)B.r, (const V *)B.r2, B.k, what, c->stream));
     return GPSS_OK;
 }
 
 // krylov! (precond = 0) / krylovPreCond! (precond = 1), krylov.jl:1-67.
 // The scalars and the stopping test live on the device (KrylovDev), so the
-// host issues iterations in chunks (2, 2, 4, 4, 8, ... up to 16) and reads the
-// solve's state back once per chunk; iterations issued past the end of the
-// solve leave phi, r and p untouched, so the result and the iteration count
-// are those of the reference's loop.
+// host issues iterations in chunks (as many as the context's last solve took,
+// at most 16, then 2, 2, 4, 4, 8, ... up to 16) and reads the solve's state back
+// once per chunk; iterations issued past the end of the solve leave phi, r and
+// p untouched, so the result and the iteration count are those of the
+// reference's loop, whatever the chunks.
 template <typename T>
 static int im_krylov(gpss_ctx *c, ImBufs &B, int scheme, double dt, void *phi, int nkrylov, double tol, int precond,
                      int *niter_out)
@@ -222,40 +226,32 @@ static int im_krylov(gpss_ctx *c, ImBufs &B, int scheme, double dt, void *phi, i
     const int64_t n = c->total;
     if (precond) {
         IM_TRY(im_mfield<T>((V *)B.s, (const V *)B.M, (const V *)B.b, n, c->stream));
-        IM_TRY(im_dot2<T>((const V *)B.s, (const V *)B.s, nullptr, nullptr, n, B.partials, B.dots, c->stream));
+        IM_TRY(im_norm2<T>((const V *)B.s, n, B.k, KRY_INIT, c->stream));
     } else {
-        IM_TRY(im_dot2<T>((const V *)B.b, (const V *)B.b, nullptr, nullptr, n, B.partials, B.dots, c->stream));
+        IM_TRY(im_norm2<T>((const V *)B.b, n, B.k, KRY_INIT, c->stream));
     }
-    IM_TRY(kry_init(B.kry, B.dots, c->stream));
     GPSS_TRY(im_apply<T>(c, B, scheme, dt, phi, true, precond, B.r));
     CUDA_TRY(c, cudaMemcpyAsync(B.r2, B.r, fb, cudaMemcpyDeviceToDevice, c->stream));
     CUDA_TRY(c, cudaMemcpyAsync(B.p, B.r, fb, cudaMemcpyDeviceToDevice, c->stream));
     KrylovDev h{};
     int issued = 0;
     for (int chunk = 0; issued < nkrylov; chunk++) {
-        const int m = std::min(chunk < 6 ? 2 << (chunk / 2) : 16, nkrylov - issued);
+        const int k = c->kry_hint > 0 ? chunk - 1 : chunk;
+        const int m = std::min(k < 0 ? c->kry_hint : k < 6 ? 2 << (k / 2) : 16, nkrylov - issued);
         for (int j = 0; j < m; j++) {
-            GPSS_TRY(im_apply<T>(c, B, scheme, dt, B.p, false, precond, B.Ap));
-            IM_TRY(im_dot2<T>((const V *)B.r, (const V *)B.r2, (const V *)B.Ap, (const V *)B.r2, n, B.partials,
-                              B.dots, c->stream));
-            IM_TRY(kry_alpha(B.kry, B.dots, c->stream));
-            IM_TRY(im_axmy_k<T>((V *)B.s, (const V *)B.r, (const V *)B.Ap, B.kry, n, c->stream));
-            GPSS_TRY(im_apply<T>(c, B, scheme, dt, B.s, false, precond, B.As));
-            IM_TRY(im_dot2<T>((const V *)B.As, (const V *)B.s, (const V *)B.As, (const V *)B.As, n, B.partials,
-                              B.dots, c->stream));
-            IM_TRY(kry_omega(B.kry, B.dots, c->stream));
-            IM_TRY(im_update_k<T>((V *)phi, (const V *)B.p, (const V *)B.s, (const V *)B.As, (V *)B.r, B.kry, n,
-                                  c->stream));
-            IM_TRY(im_dot2<T>((const V *)B.r, (const V *)B.r, (const V *)B.r, (const V *)B.r2, n, B.partials,
-                              B.dots, c->stream));
-            IM_TRY(kry_check(B.kry, B.dots, tol, nkrylov, c->stream));
-            IM_TRY(im_pdir_k<T>((V *)B.p, (const V *)B.r, (const V *)B.Ap, B.kry, n, c->stream));
+            GPSS_TRY(im_apply<T>(c, B, scheme, dt, B.p, false, precond, B.Ap, KRY_ALPHA));
+            IM_TRY(im_axmy_k<T>((V *)B.s, (const V *)B.r, (const V *)B.Ap, B.k.K, n, c->stream));
+            GPSS_TRY(im_apply<T>(c, B, scheme, dt, B.s, false, precond, B.As, KRY_OMEGA));
+            IM_TRY(im_update_k<T>((V *)phi, (const V *)B.p, (const V *)B.s, (const V *)B.As, (V *)B.r,
+                                  (const V *)B.r2, B.k, tol, nkrylov, n, c->stream));
+            IM_TRY(im_pdir_k<T>((V *)B.p, (const V *)B.r, (const V *)B.Ap, B.k.K, n, c->stream));
         }
         issued += m;
-        CUDA_TRY(c, cudaMemcpyAsync(&h, B.kry, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
+        CUDA_TRY(c, cudaMemcpyAsync(&h, B.k.K, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
         CUDA_TRY(c, cudaStreamSynchronize(c->stream));
         if (h.done) break;
     }
+    c->kry_hint = std::min(h.it, 16);
     if (h.nonfinite) return fail(c, GPSS_ENONFINITE, "Krylov solver: non-finite residual");
     *niter_out = h.niter;
     return GPSS_OK;
@@ -294,9 +290,9 @@ static int implicit_impl(gpss_ctx *c, int nsteps, int scheme, double dt, int nkr
             GPSS_TRY(im_krylov<T>(c, B, scheme, dt, B.phiw, nkrylov, tol, 1, &nk));
             total_k += nk;
             IM_TRY(im_axmy<T>((V *)B.phi1, (const V *)B.phi1, 1.0, (const V *)B.phiw, c->total, c->stream));
-            double d[2];
-            GPSS_TRY(im_dots<T>(c, B, B.phiw, B.phiw, nullptr, nullptr, d));
-            if (std::sqrt(d[0]) < tolnewton) break;
+            double d;
+            GPSS_TRY(im_norm2_host<T>(c, B, B.phiw, &d));
+            if (std::sqrt(d) < tolnewton) break;
         }
         CUDA_TRY(c, cudaMemcpyAsync(c->psi, B.phi1, fb, cudaMemcpyDeviceToDevice, c->stream));
         if (!tsch) GPSS_TRY(normalize_impl<T>(c));

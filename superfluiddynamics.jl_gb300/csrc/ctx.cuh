@@ -222,45 +222,75 @@ static int get_phase(gpss_ctx *c, int axis, double dtl, int imag, int fused, con
     const int64_t n = c->n[axis];
     const bool rot = c->omega != 0.0 && axis < 2 && c->ndim >= 2;
     const int64_t rows = rot ? (axis == 0 ? c->n[1] : c->n[0]) : 1;
-    std::vector<ldouble> re((size_t)(n * rows)), im((size_t)(n * rows));
     // fused tables of FP64 fields are fixed point (their register passes divide
     // by n, a power of two, on the way out; their generic passes want their
     // spectrum's order)
     const bool fx = fused && c->precision == GPSS_FP64, gen = fx && c->gen[axis];
-    const ldouble inv_n = fused && !(fx && !gen) ? 1.0L / (ldouble)n : 1.0L;
-    for (int64_t r = 0; r < rows; r++) {
+    // the exponent of a mode, the reference's Float64 expression: its products are
+    // rounded before they are added (a compiler that fuses one into the addition
+    // moves the exponent by an ulp)
+    auto exponent = [&](int64_t r, int64_t k) {
         const double cr = rot ? (axis == 0 ? c->coord[1][(size_t)r] : c->coord[0][(size_t)r]) : 0.0;
-        for (int64_t k = 0; k < n; k++) {
-            // the phase argument is the reference's Float64 expression; its
-            // exponential is evaluated in long double and kept as hi + lo
-            const double xk = xi_of(c, axis, k);
-            double ph;
-            if (axis == 0) ph = c->cD * (xk * xk) - c->omega * cr * xk;
-            else if (axis == 1) ph = c->cD * (xk * xk) + c->omega * cr * xk;
-            else ph = c->cD * (xk * xk);
-            ldouble fr, fi;
-            if (imag == 2) { fr = (ldouble)ph; fi = 0.0L; }  // the multiplier itself (lapRot)
-            else if (!imag) { const ldouble t = (ldouble)(ph * dtl); fr = cosl(t); fi = sinl(t); }
-            else { fr = expl((ldouble)(ph * dtl)); fi = 0.0L; }
-            re[(size_t)(r * n + k)] = fr * inv_n;
-            im[(size_t)(r * n + k)] = fi * inv_n;
-        }
-        if (gen) {
-            std::vector<ldouble> tr((size_t)n), ti((size_t)n);
-            for (int64_t p = 0; p < n; p++) {
-                const int64_t k = gen_mode_at(c->gplan[axis], (int)p);
-                tr[(size_t)p] = re[(size_t)(r * n + k)];
-                ti[(size_t)p] = im[(size_t)(r * n + k)];
-            }
-            std::copy(tr.begin(), tr.end(), re.begin() + r * n);
-            std::copy(ti.begin(), ti.end(), im.begin() + r * n);
-        }
-    }
+        const double xk = xi_of(c, axis, k);
+        volatile double p = c->cD * (xk * xk), q = c->omega * cr * xk;
+        return !rot ? p : axis == 0 ? p - q : p + q;
+    };
+    // modes k and n - k differ in the sign of xi only: without rotation their
+    // entries are the same
+    auto twin = [&](int64_t k) { return !rot && 2 * k > n ? n - k : k; };
     PhaseEntry e{axis, imag, fused, dtl, c->cD, c->omega, nullptr, rot ? (fx ? n : 2 * n) : 0};
-    if (fx) {
-        GPSS_TRY(upload_fx(c, &e.dev, fx_phase_table(re, im)));
+    bool finite = true;
+    for (int64_t r = 0; r < rows; r++)
+        for (int64_t k = 0; k < n; k++) finite = finite && std::isfinite(exponent(r, k) * dtl);
+    if (fx && !imag && finite) {
+        // real time: entries of modulus 1 (generic: 1/n, above 2^-(L + 1) for
+        // 2^L <= n), in the passes' order
+        int L = 0;
+        while (gen && (2LL << L) <= n) L++;
+        const int64_t scale = gen ? llroundl(ldexpl(1.0L / (ldouble)n, 62 + L)) : 1LL << 62;
+        std::vector<int4> t((size_t)(n * rows + 1));
+        t[0] = make_int4(-L, 0, 0, 0);
+        for (int64_t r = 0; r < rows; r++) {
+            int4 *row = &t[(size_t)(r * n + 1)];
+            std::vector<int4> nat((size_t)n);
+            for (int64_t k = 0; k < n; k++)
+                nat[(size_t)k] = twin(k) < k ? nat[(size_t)twin(k)] : fx_phase_const(exponent(r, k) * dtl, scale);
+            for (int64_t p = 0; p < n; p++) row[p] = nat[(size_t)(gen ? gen_mode_at(c->gplan[axis], (int)p) : p)];
+        }
+        GPSS_TRY(upload_fx(c, &e.dev, t));
     } else {
-        GPSS_TRY(upload_dw(c, &e.dev, re, im, rows, n));
+        std::vector<ldouble> re((size_t)(n * rows)), im((size_t)(n * rows));
+        const ldouble inv_n = fused && !(fx && !gen) ? 1.0L / (ldouble)n : 1.0L;
+        for (int64_t r = 0; r < rows; r++) {
+            for (int64_t k = 0; k < n; k++) {
+                const size_t at = (size_t)(r * n + k), tw = (size_t)(r * n + twin(k));
+                if (tw < at) {
+                    re[at] = re[tw];
+                    im[at] = im[tw];
+                    continue;
+                }
+                // the exponential is evaluated in long double and kept as hi + lo
+                const double ph = exponent(r, k);
+                ldouble fr, fi;
+                if (imag == 2) { fr = (ldouble)ph; fi = 0.0L; }  // the multiplier itself (lapRot)
+                else if (!imag) { const ldouble t = (ldouble)(ph * dtl); fr = cosl(t); fi = sinl(t); }
+                else { fr = expl((ldouble)(ph * dtl)); fi = 0.0L; }
+                re[at] = fr * inv_n;
+                im[at] = fi * inv_n;
+            }
+            if (gen) {
+                std::vector<ldouble> tr((size_t)n), ti((size_t)n);
+                for (int64_t p = 0; p < n; p++) {
+                    const int64_t k = gen_mode_at(c->gplan[axis], (int)p);
+                    tr[(size_t)p] = re[(size_t)(r * n + k)];
+                    ti[(size_t)p] = im[(size_t)(r * n + k)];
+                }
+                std::copy(tr.begin(), tr.end(), re.begin() + r * n);
+                std::copy(ti.begin(), ti.end(), im.begin() + r * n);
+            }
+        }
+        if (fx) GPSS_TRY(upload_fx(c, &e.dev, fx_phase_table(re, im)));
+        else GPSS_TRY(upload_dw(c, &e.dev, re, im, rows, n));
     }
     if (c->phases.size() > 64) {  // bounded cache: drop the oldest
         clear_graphs(c);

@@ -135,6 +135,83 @@ inline std::vector<int4> fx_phase_table(const std::vector<long double> &re, cons
     return t;
 }
 
+// exp(i theta) scale as a table constant, theta in FP64 (exact), |scale| <= 1 as
+// 2^62 scale: theta in turns from 1/(2 pi) to 128 bits, the nearest 128th of a
+// turn from a table, the rest (at most pi/128) from the Taylor series in 68-bit
+// fixed point; within 2^-63 of the exact value like the long double functions
+// it stands for, which on Arm are software (a rotating frame's tables have a row
+// per node: 64 x 48 x 56 first pass 6.8 -> 1.4 ms).  Large arguments (2^40 and
+// above) take the long double functions.
+inline int4 fx_phase_const(double theta, int64_t scale62)
+{
+    static const std::vector<int64_t> root = [] {  // exp(2 pi i k / 128) 2^68 as high part (2^62) and 6 bits
+        std::vector<int64_t> r;
+        for (int k = 0; k < 128; k++) {
+            long double v[2];
+            unit_root(k, 128, &v[0], &v[1]);
+            for (long double x : v) {
+                const int64_t hi = (int64_t)floorl(ldexpl(x, 62));
+                r.push_back(hi);
+                r.push_back((int64_t)llroundl(ldexpl(x - ldexpl((long double)hi, -62), 68)));
+            }
+        }
+        return r;
+    }();
+    using i128 = __int128;
+    using u128 = unsigned __int128;
+    auto mul = [](int64_t a, int64_t b, int shift) { return (int64_t)(((i128)a * b) >> shift); };
+    i128 re, im;  // 2^68
+    int e;
+    const double f = std::frexp(std::fabs(theta), &e);
+    if (!(f >= 0.5) && theta == 0.0) {
+        re = (i128)1 << 68;
+        im = 0;
+    } else if (e > 40) {
+        re = (i128)llroundl(ldexpl(cosl((long double)theta), 62)) << 6;
+        im = (i128)llroundl(ldexpl(sinl((long double)theta), 62)) << 6;
+    } else {
+        const uint64_t m = (uint64_t)std::ldexp(f, 53);  // |theta| = m 2^(e - 53)
+        const u128 p0 = (u128)m * 0x7f09d5f47d4d3770ULL, p1 = (u128)m * 0x28be60db9391054aULL + (p0 >> 64);
+        // |theta| / (2 pi) 2^128 = (p1 2^64 + low word of p0) 2^(e - 53), modulo 2^128
+        const uint64_t w[3] = {(uint64_t)p0, (uint64_t)p1, (uint64_t)(p1 >> 64)};
+        const int s = 53 - e;  // 13 and above: a right shift of the 192-bit product
+        auto word = [&](int i) { return i < 3 ? w[i] : (uint64_t)0; };
+        const int q = s / 64, b = s % 64;
+        const uint64_t l = b ? (word(q) >> b) | (word(q + 1) << (64 - b)) : word(q);
+        const uint64_t h = b ? (word(q + 1) >> b) | (word(q + 2) << (64 - b)) : word(q + 1);
+        u128 turns = ((u128)h << 64) | l;
+        if (theta < 0) turns = 0 - turns;
+        const int k = (int)((uint64_t)((turns + ((u128)1 << 120)) >> 121) & 127);
+        const int64_t u = (int64_t)((i128)(turns - ((u128)k << 121)) >> 58);  // 2^70 turns
+        const int64_t X = mul(u, 0x6487ed5110b4611aLL, 62);                               // radians, 2^68
+        const int64_t Z = mul(X, X, 68);
+        const int64_t one = 1LL << 62;
+        int64_t t = one / 5040 - mul(Z, one / 362880, 68);
+        t = one / 120 - mul(Z, t, 68);
+        t = one / 6 - mul(Z, t, 68);
+        const int64_t S = X - mul(X, mul(Z, t, 62), 68);  // sin
+        t = one / 720 - mul(Z, one / 40320, 68);
+        t = one / 24 - mul(Z, t, 68);
+        t = one / 2 - mul(Z, t, 68);
+        const int64_t D = mul(Z, t, 62);                  // 1 - cos
+        const int64_t *r = &root[(size_t)(4 * k)];
+        const int64_t c = r[0], n = r[2];
+        re = ((i128)c << 6) + r[1] - (((i128)c * D + (i128)n * S) >> 62);
+        im = ((i128)n << 6) + r[3] - (((i128)n * D - (i128)c * S) >> 62);
+    }
+    auto put = [&](i128 v, int &l, int &h) {  // 2^68 v scale, rounded to 2^62
+        const i128 x = scale62 == (1LL << 62) ? v : (v >> 4) * scale62 >> 58;
+        int64_t o = (int64_t)((x + 32) >> 6);
+        if ((uint32_t)o == 0x80000000u) o += o < 0 ? -1 : 1;
+        l = (int)(uint32_t)o;
+        h = (int)((o - (int64_t)l) >> 32);
+    };
+    int4 o;
+    put(re, o.x, o.y);
+    put(im, o.z, o.w);
+    return o;
+}
+
 // x / (2 pi) as m 2^e with m of 62 bits and a sign (0: m = 0)
 inline void fx_turns(long double x, int64_t &m, int &e)
 {

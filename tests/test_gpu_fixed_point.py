@@ -13,12 +13,12 @@ BOUNDS = ((0.0, 3.0), (-1.0, 4.0))
 CD, DT = -0.31, 2.3e-3
 
 
-def linear_flow(psi, shape, dtype):
+def linear_flow(psi, shape, dtype, dt=DT):
     """F^-1 exp(i cD xi^2 dt) F per axis, in the precision of dtype."""
     q = psi.astype(dtype)
     for a, (n, b) in enumerate(zip(shape, BOUNDS)):
         xi = np.fft.fftfreq(n, d=1.0 / n) * ((2 * np.pi / ((b[1] - b[0]) / n)) / n)
-        ph = (np.clongdouble(1j) * (CD * (xi * xi) * DT)).astype(dtype)
+        ph = (np.clongdouble(1j) * (CD * (xi * xi) * dt)).astype(dtype)
         q = np.fft.ifft(np.fft.fft(q, axis=a) * np.exp(ph).reshape([-1 if i == a else 1 for i in range(2)]), axis=a)
     return q
 
@@ -82,6 +82,16 @@ def test_linear_step_of_other_lengths(sfd, shape, kind):
     fp64 = rel(linear_flow(psi / scale, shape, np.complex128), exact)
     assert err < fp64 + 2.3e-16
     print(f"{kind} {shape}: {err:.2e} against {fp64:.2e} in FP64 arithmetic")
+
+
+@pytest.mark.parametrize("dt", [41.0, -3e5, 7e9])
+@pytest.mark.parametrize("shape", [(64, 32), (48, 56)])
+def test_linear_step_with_many_turns(sfd, shape, dt):
+    """Phase tables (made in integer arithmetic on the host) of arguments up to
+    1e14 radians: the bounds of the tests above."""
+    psi = field("random", shape, np.random.default_rng(3))
+    got = run_model(sfd, shape, BOUNDS, psi, coeffD=CD, beta=0.0, dt=dt, nsteps=1, precision="fp64")
+    assert rel(got, linear_flow(psi, shape, np.clongdouble, dt)) < 4 * (1.1e-16 + 0.45e-16)
 
 
 @pytest.mark.parametrize("bad", [np.nan, np.inf])

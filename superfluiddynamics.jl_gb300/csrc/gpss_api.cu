@@ -432,9 +432,6 @@ int gpss_create(gpss_ctx **out, int ndim, const int64_t *n, const double *lo, co
     c->total = 1;
     for (int a = 0; a < ndim; a++) {
         c->gen[a] = !reg_line(n[a]);
-        if (c->gen[a]) {
-            gen_plan_radices((int)n[a], c->gplan[a]);
-        }
     }
     for (int a = 0; a < 3; a++) {
         c->n[a] = a < ndim ? n[a] : 1;
@@ -448,9 +445,11 @@ int gpss_create(gpss_ctx **out, int ndim, const int64_t *n, const double *lo, co
     for (int a = 0; a < ndim; a++)
         if (c->gen[a]) {
             gen32_plan((int)n[a], c->gplan32[a]);
+            GenPlan &p = c->gplan[a];
+            Gen32Plan &q = c->gplan32[a];
+            gen_plan_field((int)n[a], c->total / n[a], a == 0, p);
             // (FP32 columns: at most 8, so that each has 16 threads for its sums)
-            c->gplan[a].lw = gen_tile_log((int)n[a], c->total / n[a], a == 0);
-            c->gplan32[a].lw = a == 0 ? c->gplan[a].lw : std::min(c->gplan[a].lw, 3);
+            q.lw = gen_tile_log(q.n, q.radix, q.nst, c->total / n[a], a == 0, a == 0 ? 6 : 3);
         }
     auto bail = [&](int rc) {
         g_create_error = c->err;

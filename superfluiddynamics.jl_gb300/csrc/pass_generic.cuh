@@ -61,9 +61,10 @@ struct GenPlan {
 
 inline bool gen_radix_is_loop(int r) { return r > 16 || r == 11 || r == 13; }
 
-// The stages of n: as few as possible, then with the smallest largest radix,
-// larger radices first; false if n has a prime factor above 31 or is too long.
-inline bool gen_plan_radices(int n, GenPlan &p)
+// The stages of n with radices up to `cap` (and prime ones above it): as few as
+// possible, then with the smallest largest radix, larger radices first; false
+// if n has a prime factor above 31 or is too long.
+inline bool gen_plan_radices(int n, GenPlan &p, int cap = 16)
 {
     p.n = n;
     p.nst = 0;
@@ -82,7 +83,8 @@ inline bool gen_plan_radices(int n, GenPlan &p)
         if (depth >= GEN_MAX_STAGES || depth + 1 > nbest) return;
         for (int i = (int)(sizeof(kRadix) / sizeof(kRadix[0])) - 1; i >= 0; i--) {
             const int r = kRadix[i];
-            if (r > top || m % r) continue;
+            const bool prime = r == 2 || r == 3 || r == 5 || r == 7 || r == 11 || r == 13 || r > 16;
+            if (r > top || m % r || (r > cap && !prime)) continue;
             cur[depth] = r;
             self(self, m / r, depth + 1, r);
         }
@@ -155,17 +157,63 @@ inline int gen_mode_at(const GenPlan &p, int pos)
     return k;
 }
 
-// Lines per tile: about 1536 cells (12 per thread), fewer while the pass has
-// under two tiles per SM -- a 2D field of 480 x 360 is 360 lines -- but at least
-// 4 adjacent columns (32 or 64 contiguous bytes) for strided lines.
-inline int gen_tile_log(int n, int64_t nlines, bool xl)
+// Lines per tile (a power of two): the thread group of a line has 128 / W
+// threads, and a stage of radix R gives each ceil(n / R / group) butterflies, so
+// a group that does not divide the butterflies leaves lanes idle (240 = 16 x 15
+// with 32 threads per line: half of them; 240^3 x pass 966 us, with 16: 700).
+// A tile's time goes with the cells of its busiest thread (a stage's barrier
+// and addresses count as two, or one where an SM has more than four tiles), c, times the tiles an SM works through -- four at
+// a time, which take 1.9 times as long as one alone (measured on fields of one to
+// four tiles per SM) -- and the W that makes that product smallest is taken, at
+// least 4 adjacent columns for strided lines (32 or 64 contiguous bytes) and
+// at most 44 KB of tile (four per SM, with their tables).  The product itself
+// goes to *time.
+inline int gen_tile_log(int n, const int *radix, int nst, int64_t nlines, bool xl, int most, double *time = nullptr)
 {
-    int lw = 0;
     const int low = xl ? 0 : 2;
-    while (lw < 6 && (n << (lw + 1)) <= 1536) lw++;
-    if (lw < low) lw = low;
-    while (lw > low && ((nlines + (1 << lw) - 1) >> lw) < 2 * 152) lw--;
-    return lw;
+    int best = low;
+    double least = 0.0;
+    for (int lw = low; lw <= most; lw++) {
+        if (lw > low && ((size_t)n << lw) * 16 > 44 * 1024) break;
+        const int group = 128 >> lw;
+        const double tiles = (double)((nlines + (1 << lw) - 1) >> lw), t = std::ceil(tiles / 152.0);
+        double c = 0.0;
+        for (int s = 0; s < nst; s++)
+            c += (double)((n / radix[s] + group - 1) / group) * radix[s] + (t <= 4.0 ? 2.0 : 1.0);
+        const double cost = c * (t <= 4.0 ? 0.7 + 0.3 * t : 1.9 * t / 4.0);
+        if (lw == low || cost < least) {
+            least = cost;
+            best = lw;
+        }
+    }
+    if (time) *time = least;
+    return best;
+}
+
+// The plan of an FP64 axis of a field: the fewest stages; or, where that leaves
+// at most four tiles per SM, of the largest radices 16, 10, 8, 6, 5 and 4 the one
+// whose tiles take the least time by the rule above.  A line of a small field
+// has more threads than butterflies of a large radix (100 = 10 x 10: 10 of 128
+// threads work), so its stages are smaller and more (100 x 100 12.4 / 14.8 -> 10.1
+// / 12.4 us); on a full chip an extra stage's products and exchanges cost more
+// than idle lanes (240^3 with 8 x 6 x 5 908 us, with 16 x 15 700).
+inline bool gen_plan_field(int n, int64_t nlines, bool xl, GenPlan &p)
+{
+    double least = 0.0;
+    bool found = false;
+    for (int cap : {16, 10, 8, 6, 5, 4}) {
+        GenPlan q;
+        if (!gen_plan_radices(n, q, cap)) continue;
+        double time;
+        q.lw = gen_tile_log(n, q.radix, q.nst, nlines, xl, 6, &time);
+        if (!found || time < least) {
+            least = time;
+            p = q;
+            found = true;
+        }
+        if (((nlines + p.lines() - 1) >> p.lw) > 4 * 152) break;
+    }
+    return found;
 }
 
 // ---- small transforms of fixed-point values ----

@@ -799,7 +799,9 @@ def run_gpss(args, rank, world, local):
             ach64 = flops_plain * v64 * 1e6 / 1e12
             fp64["roofline"] = {"bound": "fp64_fma", "unit": "TFLOP/s", "algorithmic_flops_per_cell_step": flops_plain,
                                 "achieved": ach64, "peak": peaks["fp64_tflops"], "frac": ach64 / peaks["fp64_tflops"],
-                                "peak_source": "gpss_measure_fma_rate (FP64 FMA chains, CUDA events)"}
+                                "peak_source": "gpss_measure_fma_rate (FP64 FMA chains, CUDA events)",
+                                "note": "the transforms of FP64 fields run in 64-bit fixed point on the integer "
+                                        "pipes, so the algorithmic FP64 flops are not bound by the FP64 FMA rate"}
         if other:
             other["fp32_over_fp64_plain"] = other["value"] / v64
 

@@ -447,7 +447,7 @@ int gpss_create(gpss_ctx **out, int ndim, const int64_t *n, const double *lo, co
             gen32_plan((int)n[a], c->gplan32[a]);
             GenPlan &p = c->gplan[a];
             Gen32Plan &q = c->gplan32[a];
-            gen_plan_field((int)n[a], c->total / n[a], a == 0, p);
+            if (precision == GPSS_FP64) gen_plan_field((int)n[a], c->total / n[a], a == 0, p);
             // (FP32 columns: at most 8, so that each has 16 threads for its sums)
             q.lw = gen_tile_log(q.n, q.radix, q.nst, c->total / n[a], a == 0, a == 0 ? 6 : 3);
         }

@@ -198,7 +198,8 @@ __device__ __forceinline__ double2 nl_apply(double2 v, double Vv, const NLConst<
 // The same in imaginary time for the passes of FP64 fields, of psi = scale v:
 // exp(-(V + beta |psi|^2) dt) psi.  The exponential runs on the integer pipes
 // (fx_exp2neg), its argument in units of ln 2 with 1/ln 2 as hi + lo; eight
-// FP64 operations per cell remain.
+// FP64 operations per cell remain.  A wall (V = +inf) takes the hi part alone:
+// the lo part has either sign, and inf - inf would be NaN where exp gives 0.
 struct NLImag64 {
     double b2, dh, dl, s;
     const long long *tab2;
@@ -211,7 +212,8 @@ struct NLImag64 {
     __device__ __forceinline__ double2 operator()(double2 v, double Vv) const
     {
         const double r = fma(b2, fma(v.x, v.x, v.y * v.y), Vv);
-        const double f = s * fx_exp2neg(fma(r, dh, r * dl), tab2);
+        const bool finite = (__double2hiint(r) & 0x7ff00000) != 0x7ff00000;
+        const double f = s * fx_exp2neg(fma(r, dh, finite ? r * dl : 0.0), tab2);
         return make_double2(f * v.x, f * v.y);
     }
 };

@@ -25,7 +25,7 @@ using namespace gpss;
 static const double kTwoPi = 6.283185307179586;  // Float64(2pi)
 
 struct PhaseEntry {
-    int axis, imag, fused;
+    int axis, imag, fused, mult;  // mult: a multiplier table (FP64)
     double dtl, cD, om;
     void *dev;
     int64_t prow;
@@ -209,13 +209,14 @@ static void clear_graphs(gpss_ctx *c);
 // 1/n of the inverse transform.  With Omega != 0 the x (y) table has one row
 // per y (x) node.
 static int get_phase(gpss_ctx *c, int axis, double dtl, int imag, int fused, const void **dev,
-                     int64_t *prow)
+                     int64_t *prow, int *mult = nullptr)
 {
     for (auto &e : c->phases) {
         if (e.axis == axis && e.dtl == dtl && e.imag == imag && e.fused == fused && e.cD == c->cD &&
             e.om == c->omega) {
             *dev = e.dev;
             *prow = e.prow;
+            if (mult) *mult = e.mult;
             return GPSS_OK;
         }
     }
@@ -238,10 +239,18 @@ static int get_phase(gpss_ctx *c, int axis, double dtl, int imag, int fused, con
     // modes k and n - k differ in the sign of xi only: without rotation their
     // entries are the same
     auto twin = [&](int64_t k) { return !rot && 2 * k > n ? n - k : k; };
-    PhaseEntry e{axis, imag, fused, dtl, c->cD, c->omega, nullptr, rot ? (fx ? n : 2 * n) : 0};
-    bool finite = true;
+    PhaseEntry e{axis, imag, fused, 0, dtl, c->cD, c->omega, nullptr, rot ? (fx ? n : 2 * n) : 0};
+    bool finite = true, decays = true;
     for (int64_t r = 0; r < rows; r++)
-        for (int64_t k = 0; k < n; k++) finite = finite && std::isfinite(exponent(r, k) * dtl);
+        for (int64_t k = 0; k < n; k++) {
+            finite = finite && std::isfinite(exponent(r, k) * dtl);
+            decays = decays && exponent(r, k) * dtl <= 0.0;
+        }
+    // multipliers of any size: a significand and an exponent per entry.  Factors
+    // of at most 1, the largest of them that of k = 0 where the field's weight
+    // is, lose nothing on one exponent, and the merged imaginary-time passes take
+    // no other table.
+    e.mult = fx && (imag == 2 || (imag == 1 && !decays));
     if (fx && !imag && finite) {
         // real time: entries of modulus 1 (generic: 1/n, above 2^-(L + 1) for
         // 2^L <= n), in the passes' order
@@ -289,7 +298,7 @@ static int get_phase(gpss_ctx *c, int axis, double dtl, int imag, int fused, con
                 std::copy(ti.begin(), ti.end(), im.begin() + r * n);
             }
         }
-        if (fx) GPSS_TRY(upload_fx(c, &e.dev, fx_phase_table(re, im)));
+        if (fx) GPSS_TRY(upload_fx(c, &e.dev, e.mult ? fx_mult_table(re) : fx_phase_table(re, im)));
         else GPSS_TRY(upload_dw(c, &e.dev, re, im, rows, n));
     }
     if (c->phases.size() > 64) {  // bounded cache: drop the oldest
@@ -301,6 +310,7 @@ static int get_phase(gpss_ctx *c, int axis, double dtl, int imag, int fused, con
     c->phases.push_back(e);
     *dev = e.dev;
     *prow = e.prow;
+    if (mult) *mult = e.mult;
     return GPSS_OK;
 }
 
@@ -598,7 +608,7 @@ static int kinetic_fused(gpss_ctx *c, double dtl, int imag, bool nl, double dtnl
         const int axis = reverse ? c->ndim - 1 - step : step;
         PassArgs<T> a = axis_args<T>(c, axis, field, field);
         const void *ph;
-        GPSS_TRY(get_phase(c, axis, dtl, imag, 1, &ph, &a.prow));
+        GPSS_TRY(get_phase(c, axis, dtl, imag, 1, &ph, &a.prow, &a.mult));
         a.phase = (const vec2<T> *)ph;
         a.comp = sizeof(T) == 4 && (c->flags & GPSS_FLAG_COMPENSATED) != 0;
         // the FP32 mass lock holds the field at the target mass M0 (its

@@ -91,6 +91,43 @@ __device__ __forceinline__ fxc fx_quarter(fxc a)
     return fxc{(a.x + 2) >> 2, (a.y + 2) >> 2};
 }
 
+// ---- multipliers: real factors of a spectrum that differ by orders of magnitude
+//
+// A multiplier pass (the Laplacian's (2 pi k / L)^2, an imaginary-time factor
+// above 1) does not keep the line's norm, and its largest factor belongs to
+// modes that hardly carry weight: on the quantum that this factor asks for, the
+// low modes would be held in 2 log2(n / 2) bits less.  So each table entry has a
+// 62-bit significand and its own exponent {low half, high half, exponent less the
+// table's, 0}, and a line takes a new quantum from the 2-norm of its products
+// (gen_pass_kernel and pass_kernel: one more reduction per line; 64^3 explicit
+// Runge-Kutta, 8 steps, 2102 -> 2141 us; backward Euler, a step, 64^3 211 -> 215,
+// 256^3 7120 -> 7560 us).
+
+// a times the significand / 4
+__device__ __forceinline__ fxc fx_mult(fxc a, int4 m) { return fxc{fx_rmul(a.x, m.y, m.x), fx_rmul(a.y, m.y, m.x)}; }
+// the square of |a 2^e| 2^-20, e at most 0
+__device__ __forceinline__ float fx_mult_norm2(fxc a, int e)
+{
+    const float f = __int_as_float((127 + max(e - 20, -126)) << 23);
+    const float x = (float)a.x * f, y = (float)a.y * f;
+    return fmaf(x, x, y * y);
+}
+// the exponent by which a line whose products have the sum of squares s (as
+// above) is shifted down so that its 2-norm takes `bits` bits; below 2^-100 the
+// products are rounding of zeros
+__device__ __forceinline__ int fx_mult_shift(float s, int bits)
+{
+    const int es = (__float_as_int(fmaxf(s, 7.8886e-31f)) >> 23) - 127;  // s < 2^(es + 1)
+    return ((es + 2) >> 1) + 20 - bits;
+}
+// v 2^s, rounded
+__device__ __forceinline__ long long fx_scale2(long long v, int s)
+{
+    const int r = min(max(-s, 0), 62);
+    return ((v << min(max(s, 0), 63)) + ((1LL << r) >> 1)) >> r;
+}
+__device__ __forceinline__ fxc fx_scale2(fxc a, int s) { return fxc{fx_scale2(a.x, s), fx_scale2(a.y, s)}; }
+
 // the DFT-16's own constants as 2^64 times a number below 1/2, signed halves
 constexpr long long FX_TAN16 = 0x32ebebc0aa62b00fLL;   // tan(pi/16)
 constexpr long long FX_SIN8 = 0x61f78a9abaa58b47LL;    // sin(pi/8)

@@ -97,7 +97,7 @@ static int imag_flow(gpss_ctx *c, double dtl, const void *in0, bool pre_nl, void
         const bool first = axis == 0, last = axis == c->ndim - 1;
         PassArgs<T> a = axis_args<T>(c, axis, first ? in0 : c->psi, last ? out_last : c->psi);
         const void *ph;
-        GPSS_TRY(get_phase(c, axis, dtl, 1, 1, &ph, &a.prow));
+        GPSS_TRY(get_phase(c, axis, dtl, 1, 1, &ph, &a.prow, &a.mult));
         a.phase = (const vec2<T> *)ph;
         if ((first && pre_nl) || (last && nl_last)) GPSS_TRY(set_nl<T>(c, a, NL_NONE, dtnl, false));
         if (first && pre_nl) {
@@ -296,7 +296,9 @@ static int step_impl(gpss_ctx *c, int nsteps, int scheme, int imag, double dt, g
             c->pending_scale = lock;
         }
     } else if (imag && scheme == GPSS_STRANG && c->omega == 0.0 && !(c->flags & GPSS_FLAG_NOMERGE) &&
-               (sizeof(T) == 8 || !any_generic(c))) {
+               (sizeof(T) == 8 ? c->cD * dt <= 0.0 : !any_generic(c))) {
+        // (FP64 factors that grow are multiplier tables, which the merged passes
+        // do not take)
         GPSS_TRY(imag_merged<T>(c, nsteps, dt));
     } else if (imag) {
         for (int s = 0; s < nsteps; s++) {

@@ -1,6 +1,8 @@
 // gpss_internal.h -- declarations shared by the translation units of libgpss.
 #pragma once
 #include <cuda_runtime.h>
+#include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -109,7 +111,7 @@ inline std::vector<int4> fx_table(const std::vector<long double> &re, const std:
     for (size_t i = 0; i < t.size(); i++) t[i] = fx_const(re[i], im[i]);
     return t;
 }
-// A fixed-point phase or multiplier table: a leading entry with the exponent e,
+// A fixed-point table of phases or decaying factors: a leading entry with the exponent e,
 // then the values divided by 2^e, the smallest power of two at or above their
 // largest modulus.  A non-finite value makes every result of a pass with the
 // table NaN or infinite in FP64; here its exponent overflows the pass's result.
@@ -132,6 +134,29 @@ inline std::vector<int4> fx_phase_table(const std::vector<long double> &re, cons
     t[0] = make_int4(finite ? e : 1 << 20, 0, 0, 0);
     for (size_t i = 0; i < re.size(); i++)
         t[i + 1] = finite ? fx_const(ldexpl(re[i], -e), ldexpl(im[i], -e)) : fx_const(1.0L, 0.0L);
+    return t;
+}
+
+// A multiplier table (fft_fix.cuh): a leading entry with the exponent e of the
+// largest value, then per value a 62-bit significand as halves and its exponent
+// less e.  Non-finite values as above.
+inline std::vector<int4> fx_mult_table(const std::vector<long double> &v)
+{
+    std::vector<int4> t(v.size() + 1, make_int4(0, 1 << 30, 0, 0));
+    int top = INT_MIN;
+    for (size_t i = 0; i < v.size(); i++) {
+        if (!std::isfinite((double)v[i])) {
+            std::fill(t.begin(), t.end(), make_int4(0, 1 << 30, 0, 0));
+            t[0] = make_int4(1 << 20, 0, 0, 0);
+            return t;
+        }
+        int e = 0;
+        fx_halves(frexpl(v[i], &e), t[i + 1].x, t[i + 1].y);
+        t[i + 1].z = e;
+        if (v[i] != 0.0L) top = std::max(top, e);
+    }
+    t[0] = make_int4(top == INT_MIN ? 0 : top, 0, 0, 0);
+    for (size_t i = 0; i < v.size(); i++) t[i + 1].z = v[i] != 0.0L ? t[i + 1].z - t[0].x : 0;
     return t;
 }
 

@@ -135,6 +135,14 @@ static cudaError_t launch_pass_sized(int mode, const PassArgs<T> &a, int blocks,
         if (sizeof(T) == 8 && a.nl_mode == NL_REAL && a.scale) return cudaErrorInvalidValue;
         if (sizeof(T) == 8 && (a.nl_mode != NL_NONE || a.nl_pre || a.adj_pre) && !a.nl_fx.tab2)
             return cudaErrorInvalidValue;
+        // multiplier tables: the accumulating instantiation (which takes no
+        // others) or the full one
+        if constexpr (sizeof(T) == 8) {
+            if (a.mult && (a.nl_pre || a.dot_with)) return cudaErrorInvalidValue;
+            if (a.mult && !diag && !adj && !nl)
+                return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_ACC | SIZE>(a, blocks, s);
+            if (a.mult || acc) return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_ALL | SIZE>(a, blocks, s);
+        }
         if (a.nl_pre || a.dot_with) {
             if (diag || acc || adj || a.nl_mode != NL_NONE) return cudaErrorInvalidValue;
             return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_IMAGM | SIZE>(a, blocks, s);
@@ -154,7 +162,9 @@ static cudaError_t launch_pass_sized(int mode, const PassArgs<T> &a, int blocks,
             }
         }
         if (diag || (acc && (adj || nl))) return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_ALL | SIZE>(a, blocks, s);
-        if (acc) return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_ACC | SIZE>(a, blocks, s);
+        if constexpr (sizeof(T) == 4) {
+            if (acc) return launch_pass_inst<T, N, XL, MODE_FUSED, FEAT_ACC>(a, blocks, s);
+        }
         if constexpr (sizeof(T) == 4 && !XL && N >= 64) {
             // fewer default tiles than SMs: the 128-thread y/z instantiation
             if (blocks < sm_count()) {

@@ -55,6 +55,7 @@ struct GenPlan {
     // with the spectrum has its own); and the resulting exponents
     int kf[GEN_MAX_STAGES], kp, kb[GEN_MAX_STAGES], ki[GEN_MAX_STAGES];
     int bits_f, bits_i;           // the line's 2-norm takes this many bits
+    int bits_p;                   // and may take this many after the phase
     int ef, et, ei;               // exponent of the spectrum, the result, the inverse alone
     int lines() const { return 1 << lw; }
 };
@@ -132,6 +133,7 @@ inline bool gen_plan_radices(int n, GenPlan &p, int cap = 16)
             }
             espec = e;
             p.kp = product(p.radix[S - 1]);
+            p.bits_p = (int)std::floor(b + 1e-9);
         }
         step(p.radix[S - 1]);
         for (int s = S - 2; s >= 0; s--) {
@@ -411,7 +413,8 @@ __device__ __noinline__ void gen_stage_loop(const GenPlan &p, int s, int kind, i
     }
 }
 
-template <int MODE>
+// MULT: the phase is a multiplier table (fft_fix.cuh)
+template <int MODE, bool MULT = false>
 __global__ void __launch_bounds__(GEN_THREADS, 4)
 gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
 {
@@ -427,8 +430,9 @@ gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
     const bool rowph = MODE == MODE_FUSED && a.prow != 0;
     const bool mask = MODE == MODE_FUSED && a.mask_lim != nullptr;
     fxc *data = reinterpret_cast<fxc *>(sph + (MODE == MODE_FUSED && !rowph && !mask ? n : 0));
-    __shared__ int sword[64];
-    __shared__ unsigned ssum[64];
+    static_assert(!MULT || MODE == MODE_FUSED, "multipliers: fused passes");
+    __shared__ int sword[64], smword[64];    // (m: of the multiplied spectrum)
+    __shared__ unsigned ssum[64], smsum[64];
     const int tid = threadIdx.x;
     // a thread's line, its first position and its stride over the positions
     const int lstep = 7 - lw, step = 1 << lstep;
@@ -478,6 +482,10 @@ gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
         if (i0 == 0) {
             sword[w] = 0;
             ssum[w] = 0u;
+            if (MULT) {
+                smword[w] = 0;
+                smsum[w] = 0u;
+            }
         }
         float top = 0.f;  // the largest upper word
 #pragma unroll 4
@@ -543,6 +551,9 @@ gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
         const int4 *ph = rowph ? gphase + (int64_t)row * a.prow : sph;
         (void)lim;
         (void)ph;
+        float s2 = 0.f;  // MULT: this thread's sum of squares
+        int qm = 0;      // and the exponent that the products' quantum adds
+        (void)s2;
         auto spectral = [&](fxc &u, int pos) {
             if constexpr (MODE == MODE_FUSED || MODE == MODE_DIAG) {
                 if (red & RED_KIN) {
@@ -554,7 +565,11 @@ gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
                     if (a.coord) acc_rot += xi * m2 * (T)(1.0 / n) * (T)a.coord[row];
                 }
             }
-            if constexpr (MODE == MODE_FUSED) {
+            if constexpr (MULT) {
+                const int4 t = ph[pos];
+                u = fx_mult(u, t);
+                s2 += fx_mult_norm2(u, t.z);
+            } else if constexpr (MODE == MODE_FUSED) {
                 if (mask) {
                     const int k = mode_at[pos], kk = k < (n + 1) / 2 ? k : n - k;
                     u = kk <= lim ? gen_shift(fx_quarter(u), p.kp) : fxc{0, 0};
@@ -567,15 +582,18 @@ gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
         // ---- the stages
         const int S = p.nst;
         const int *kb = kFwd ? p.kb : p.ki;
+        // (MULT: the middle stage is two, with the products' quantum between them)
+        const int mid2 = MULT ? S : S - 1;
 #pragma unroll 1
-        for (int it = kFwd ? 0 : S - 1; it < (kBwd ? 2 * S - 1 : S); it++) {
-            const int s = it < S ? it : 2 * S - 2 - it;
-            const int kind = it < S - 1 ? GEN_FWD : it == S - 1 ? GEN_MID : GEN_BWD;
+        for (int it = kFwd ? 0 : S - 1; it < (kBwd ? mid2 + S : S); it++) {
+            const int s = it < S ? it : mid2 + S - 1 - it;
+            const int kind = it < S - 1 ? GEN_FWD : it <= mid2 ? GEN_MID : GEN_BWD;
             const int *sh = kind == GEN_FWD ? p.kf : kb;
+            const bool fwd = kFwd && (!MULT || it < S), bwd = kBwd && (!MULT || it >= S);
             tile_sync();
             auto run = [&](auto radix) {
                 constexpr int R = decltype(radix)::value;
-                gen_stage<R>(p, s, kind, i0, step, kFwd, kBwd, roots, sh, data, at, [&](fxc *u, int p0) {
+                gen_stage<R>(p, s, kind, i0, step, fwd, bwd, roots, sh, data, at, [&](fxc *u, int p0) {
 #pragma unroll
                     for (int i = 0; i < R; i++) spectral(u[i], p0 + i);
                 });
@@ -594,8 +612,27 @@ gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
             case 15: run(std::integral_constant<int, 15>{}); break;
             case 16: run(std::integral_constant<int, 16>{}); break;
             default:
-                gen_stage_loop(p, s, kind, i0, step, kFwd, kBwd, roots, sh, data, at, spectral);
+                gen_stage_loop(p, s, kind, i0, step, fwd, bwd, roots, sh, data, at, spectral);
                 break;
+            }
+            if constexpr (MULT) {
+                if (it == S - 1) {
+                    // the sum over the line's threads in whole units of 2^-16 of
+                    // their largest sum's exponent
+                    tile_sync();
+                    atomicMax(&smword[w], __float_as_int(s2));
+                    tile_sync();
+                    const int e = min(smword[w] >> 23, 250);
+                    atomicAdd(&smsum[w], (unsigned)(s2 * __int_as_float((254 - e) << 23) * 65536.f) + 1u);
+                    tile_sync();
+                    qm = fx_mult_shift((float)smsum[w] * __int_as_float(max(e - 16, 1) << 23), p.bits_p);
+                    for (int i = i0; i < n; i += step) {
+                        const int slot = at(i);
+                        const fxc u = fx_scale2(data[slot], ph[i].z - qm);
+                        data[slot] = fxc{u.y, u.x};
+                    }
+                    qm += p.kp;
+                }
             }
         }
         tile_sync();
@@ -607,7 +644,7 @@ gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
             }
         }
         if constexpr (MODE == MODE_FUSED || MODE == MODE_INV) {
-            int qv = q + (MODE == MODE_FUSED ? p.et + fxpe : p.ei), lsh = 0, rsh = 0;
+            int qv = q + (MODE == MODE_FUSED ? p.et + fxpe + qm : p.ei), lsh = 0, rsh = 0;
             if (fxnl) {
                 const int sh = 190 + 2 * qv + a.nl_fx.ge;
                 lsh = min(max(sh, 0), 63);

@@ -92,7 +92,8 @@ enum { NL_NONE = 0, NL_REAL = 1, NL_IMAG = 2 };
 //              axis of a spectrum already transformed along the others, keep
 //              the modes with |kk| <= mask_lim[line] (scaled by 1/n), zero the rest
 //   FEAT_ACC   the `acc` epilogue alone (add the result to a second field:
-//              the y/z passes of lapRot in the RK and implicit schemes)
+//              the y/z passes of lapRot in the RK and implicit schemes); FP64:
+//              all its passes, with their multiplier tables
 //   FEAT_COMP  (FP32) compensated arithmetic: the transforms, twiddles and
 //              phase run on grid-exact two-float values (fft_comp.cuh), so
 //              the only FP32 rounding of the pass is the store; combined with
@@ -151,6 +152,7 @@ template <typename T> struct PassArgs {
     double nl_beta, nl_dt;
     NLSplit nl_split;        // FP32 kernels: beta, dt, beta*dt as float pairs
     FxNlArgs nl_fx;          // FP64 register passes, real time: the flow in fixed point
+    int mult;                // FP64: `phase` is a multiplier table (fft_fix.cuh)
     // deferred renormalisation: multiply the input by the factor in a
     // ScaleCell (nullable; `scale` points at its FP64 member)
     const double *scale;
@@ -716,7 +718,7 @@ pass_kernel(const PassArgs<T> a)
 
     if constexpr (kFix) {
         // FP64 field: the same stages on 64-bit fixed-point values.  The tile's
-        // lines each take their quantum from their largest component.
+        // lines each take their quantum from their 2-norm.
         constexpr int NI = N1 / N2;
         // radix-4 stages: the natural-order mode of value i of this thread, whose
         // positions 4 r + i follow the digits of the stages (4, 4, .. and a last
@@ -854,6 +856,45 @@ pass_kernel(const PassArgs<T> a)
         const int4 *phrow = prow ? fxph + row * prow : sph;
         (void)phrow;
         (void)spectrum;
+        // multiplier tables (accumulating passes have no others): the line's
+        // products, then their common quantum
+        constexpr bool kMult = MODE == MODE_FUSED && kAcc && !kMask && !kImagM;
+        const bool mult = kMult && (!kDiag || a.mult);
+        constexpr int kMultBits = kQuad ? 61 : 60;
+        int qm = 0;  // the exponent that the products' quantum adds
+        auto line_sum = [&](float s) {
+#pragma unroll
+            for (int o = XL ? (P < 32 ? P : 32) / 2 : 16; o >= (XL ? 1 : W); o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if constexpr (kMult && (XL ? P > 32 : P > 1)) {
+                // (read before the barrier ahead of the next stage, written
+                // again by the next tile after it)
+                __shared__ float part[THREADS];
+                constexpr int G = XL ? P / 32 : W < 32 ? THREADS / 32 : P;
+                if (XL ? (tid & 31) == 0 : W >= 32 || (tid & 31) < W)
+                    part[XL ? tid >> 5 : W < 32 ? (tid >> 5) * W + w : tid] = s;
+                __syncthreads();
+                s = 0.f;
+#pragma unroll
+                for (int i = 0; i < G; i++) s += part[XL ? w * G + i : i * W + w];
+            }
+            return s;
+        };
+        auto times_mult = [&](auto &u, auto count, auto mode) {  // value i of u is mode(i)
+            constexpr int M = decltype(count)::value;
+            float s = 0.f;
+#pragma unroll
+            for (int i = 0; i < M; i++) {
+                const int4 t = phrow[mode(i)];
+                u[i] = fx_mult(u[i], t);
+                s += fx_mult_norm2(u[i], t.z);
+            }
+            qm = fx_mult_shift(line_sum(s), kMultBits);
+#pragma unroll
+            for (int i = 0; i < M; i++) u[i] = fx_scale2(u[i], phrow[mode(i)].z - qm);
+        };
+        (void)mult;
+        (void)line_sum;
+        (void)times_mult;
         using cN1 = std::integral_constant<int, N1>;
         using cN2 = std::integral_constant<int, N2>;
         using c1 = std::integral_constant<int, 1>;
@@ -920,7 +961,10 @@ pass_kernel(const PassArgs<T> a)
                         for (int i = 0; i < 4; i++) a.out[base + (uint32_t)quad_mode(i) * st] = os(c[i], false);
                     }
                 }
-                if constexpr (MODE == MODE_FUSED) {
+                if (kMult && mult) {
+                    if constexpr (kMult) times_mult(c, cN1{}, quad_mode);
+                    qm += 1;  // (its products are not doubled)
+                } else if constexpr (MODE == MODE_FUSED) {
                     const int lim = kMask ? a.mask_lim[gg] : 0;
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
@@ -966,9 +1010,12 @@ pass_kernel(const PassArgs<T> a)
                 if (it == 0) {
                     spectrum(c, cN1{}, 0, c1{});
                     if constexpr (MODE == MODE_FUSED) {
+                        if constexpr (kMult) {
+                            if (mult) times_mult(c, cN1{}, [](int i) { return i; });
+                        }
 #pragma unroll
                         for (int j = 0; j < N1; j++) {
-                            if constexpr (!kMask) c[j] = fx_cmul(c[j], phrow[j]);
+                            if (!kMask && !mult) c[j] = fx_cmul(c[j], phrow[j]);
                             exchange(c[j]);
                         }
                     }
@@ -997,7 +1044,10 @@ pass_kernel(const PassArgs<T> a)
                 }
                 dft<N1, -1>(c);
                 if (it == 1) spectrum(c, cN1{}, r, cN2{});
-                if (it < 3 && !(it == 1 && (kSpecOnly || kMask))) {
+                if constexpr (kMult) {
+                    if (it == 1 && mult) times_mult(c, cN1{}, [&](int i) { return r + N2 * i; });
+                }
+                if (it < 3 && !(it == 1 && (kSpecOnly || kMask || mult))) {
                     const int4 *tab = (it == 1 ? phrow : stw) + r;
 #pragma unroll
                     for (int j = 0; j < N1; j++) c[j] = fx_cmul(c[j], tab[j * N2]);
@@ -1059,7 +1109,40 @@ pass_kernel(const PassArgs<T> a)
                             for (int rr = 0; rr < N2; rr++) sfx[sidx(k1 * N2 + rr)] = u[rr];
                         }
                     };
-                    if constexpr (MODE == MODE_INV) {
+                    if (kMult && mult) {
+                        // the products of all items, their quantum, the way back
+                        if constexpr (kMult) {
+                            float s = 0.f;
+                            fxc u[N2];
+#pragma unroll 1
+                            for (int k1 = r; k1 < N1; k1 += P) {
+#pragma unroll
+                                for (int rr = 0; rr < N2; rr++) u[rr] = sfx[sidx(k1 * N2 + rr)];
+                                dft<N2, -1>(u);
+                                spectrum(u, cN2{}, k1, cN1{});
+#pragma unroll
+                                for (int k2 = 0; k2 < N2; k2++) {
+                                    const int4 t = phrow[k1 + N1 * k2];
+                                    u[k2] = fx_mult(u[k2], t);
+                                    s += fx_mult_norm2(u[k2], t.z);
+                                    sfx[sidx(k1 * N2 + k2)] = u[k2];
+                                }
+                            }
+                            qm = fx_mult_shift(line_sum(s), kMultBits);
+#pragma unroll 1
+                            for (int k1 = r; k1 < N1; k1 += P) {
+#pragma unroll
+                                for (int k2 = 0; k2 < N2; k2++) {
+                                    u[k2] = fx_scale2(sfx[sidx(k1 * N2 + k2)], phrow[k1 + N1 * k2].z - qm);
+                                    exchange(u[k2]);
+                                }
+                                dft<N2, -1>(u);
+#pragma unroll
+                                for (int k2 = 0; k2 < N2; k2++)
+                                    sfx[sidx(k1 * N2 + k2)] = fx_cmul(u[k2], stwB[k1 + N1 * k2]);
+                            }
+                        }
+                    } else if constexpr (MODE == MODE_INV) {
                         item(r, std::integral_constant<int, 0>{});
                         if constexpr (NI > 1) item(r + P, std::integral_constant<int, 1>{});
                         static_assert(NI <= 2, "two items per thread at most");
@@ -1082,7 +1165,7 @@ pass_kernel(const PassArgs<T> a)
         }
         if constexpr (MODE == MODE_FUSED || MODE == MODE_INV) {
             // 1/n of the inverse, and the deferred factor
-            int qv = qo - FxLog<N>::V;
+            int qv = qo + qm - FxLog<N>::V;
             if constexpr (MODE == MODE_FUSED && kNL) {
                 if (fxnl) {
                     if constexpr (kAdj) {

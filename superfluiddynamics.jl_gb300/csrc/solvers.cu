@@ -77,7 +77,7 @@ template <typename T> static int lap_rot_dev(gpss_ctx *c, const void *q, void *o
     for (int axis = 0; axis < c->ndim; axis++) {
         PassArgs<T> a = axis_args<T>(c, axis, q, out);
         const void *ph;
-        GPSS_TRY(get_phase(c, axis, 0.0, 2, 1, &ph, &a.prow));
+        GPSS_TRY(get_phase(c, axis, 0.0, 2, 1, &ph, &a.prow, &a.mult));
         a.phase = (const vec2<T> *)ph;
         if (axis > 0) a.acc = (const vec2<T> *)out;
         GPSS_TRY(launch<T>(c, axis, MODE_FUSED, a));

@@ -76,16 +76,11 @@ struct gpss_ctx {
     int *status = nullptr;    // [1]
     unsigned int *counter = nullptr;  // arrival counter of the in-kernel reduction finish
     std::vector<PhaseEntry> phases;
-    // FP64 fields: what the fixed-point nonlinear flow reads besides the field
-    // -- roots of unity, and per time step V dt in turns (set_nl); vbad: V
-    // holds NaN or infinity
-    struct VturnEntry {
-        double dt;
-        void *dev;
-    };
-    std::vector<VturnEntry> vturns;
-    void *nl_tab = nullptr;
-    int *vbad = nullptr;
+    void *nl_tab = nullptr;  // FP64 fields: the nonlinear flow's roots of unity and powers of two
+    // its factors of the last beta and dt (long double quotients, software on Arm,
+    // and asked for at each launch that is not replayed from a graph)
+    double nl_beta = 0.0, nl_dt = 0.0;
+    FxNlArgs nl_fx{};
     void *rk_buf[4] = {nullptr, nullptr, nullptr, nullptr};  // RK: stage state, lapRot, NL term, sum
     int *rk_lim = nullptr;    // RK: 2/3-rule limits per inner position (the FEAT_MASK pass)
     void *im_buf = nullptr;   // implicit schemes: work fields (implicit_impl)
@@ -391,48 +386,6 @@ static std::string graph_key(const char *what, std::initializer_list<double> v)
 static const int64_t kGraphCells = int64_t(1) << 21;
 static const int kGraphChunk = 32;  // time steps per captured chunk
 
-// The table V dt / (2 pi) of a time step (fft_fix.cuh), made on its first use
-// after the potential was set.  Graphs hold its address, so the tables of up
-// to four time steps are kept (a program that alternates between two finds
-// both); a fifth takes the place of the oldest, and the graphs go.
-static int get_vturn(gpss_ctx *c, double dt, const long long **dev)
-{
-    for (auto &e : c->vturns)
-        if (e.dt == dt) {
-            *dev = (const long long *)e.dev;
-            return GPSS_OK;
-        }
-    void *buf = nullptr;
-    if (c->vturns.size() >= 4) {
-        clear_graphs(c);  // the stream orders the overwrite behind earlier launches
-        buf = c->vturns.front().dev;
-        c->vturns.erase(c->vturns.begin());
-    } else {
-        GPSS_TRY(dev_alloc(c, &buf, (size_t)c->total * sizeof(long long)));
-    }
-    c->vturns.push_back({dt, buf});
-    int64_t m;
-    int e;
-    fx_turns((ldouble)dt, m, e);
-    CUDA_TRY(c, launch_vturn((const double *)c->V, (long long *)buf, m, e, c->total, c->vbad, c->stream));
-    c->launches++;
-    *dev = (const long long *)buf;
-    return GPSS_OK;
-}
-
-// forget the tables of the previous potential (their buffers are freed)
-static void clear_vturns(gpss_ctx *c)
-{
-    if (c->vturns.empty()) return;
-    clear_graphs(c);
-    if (c->stream) cudaStreamSynchronize(c->stream);
-    for (auto &e : c->vturns) {
-        cudaFree(e.dev);
-        c->bytes -= (int64_t)((size_t)c->total * sizeof(long long));
-    }
-    c->vturns.clear();
-}
-
 // the nonlinear flow N(dt) of a pass: its epilogue (mode), or with NL_NONE the
 // constants of a prologue (imaginary time) or of the flow's adjoint (real_time)
 template <typename T> static int set_nl(gpss_ctx *c, PassArgs<T> &a, int mode, double dt, bool real_time)
@@ -460,23 +413,22 @@ template <typename T> static int set_nl(gpss_ctx *c, PassArgs<T> &a, int mode, d
         }();
         GPSS_TRY(upload_fx(c, &c->nl_tab, table));
     }
+    if (real_time) {
+        if (c->nl_beta != c->beta || c->nl_dt != dt) {
+            FxNlArgs &f = c->nl_fx;
+            int64_t m;
+            fx_turns((ldouble)c->beta * (ldouble)dt, m, f.ge);
+            f.gl = (int)(uint32_t)m;
+            f.gh = (int)((m - (int64_t)f.gl) >> 32);
+            fx_turns((ldouble)dt, m, f.de);
+            f.d = m;
+            c->nl_beta = c->beta;
+            c->nl_dt = dt;
+        }
+        a.nl_fx = c->nl_fx;
+    }
     a.nl_fx.tab = (const int4 *)c->nl_tab;
     a.nl_fx.tab2 = (const long long *)(a.nl_fx.tab + FX_NL_TAB);
-    if (!real_time) return GPSS_OK;
-    int64_t m;
-    int e;
-    fx_turns((ldouble)c->beta * (ldouble)dt, m, e);
-    a.nl_fx.gl = (int)(uint32_t)m;
-    a.nl_fx.gh = (int)((m - (int64_t)a.nl_fx.gl) >> 32);
-    a.nl_fx.ge = e;
-    if (c->have_V) {
-        if (!c->vbad) {
-            GPSS_TRY(dev_alloc(c, (void **)&c->vbad, sizeof(int)));
-            CUDA_TRY(c, cudaMemsetAsync(c->vbad, 0, sizeof(int), c->stream));
-        }
-        GPSS_TRY(get_vturn(c, dt, &a.nl_fx.vturn));
-        a.nl_fx.vbad = c->vbad;
-    }
     return GPSS_OK;
 }
 

@@ -262,18 +262,18 @@ __device__ __forceinline__ double fx_double(long long v, int q)
 // psi <- exp(-i theta) psi with theta = (V + beta |psi|^2) dt in turns, as a
 // 64-bit fraction whose overflow is the reduction modulo one turn: |psi|^2
 // from the integers, times beta dt / 2 pi (63 bits and an exponent), plus V dt
-// / 2 pi from a table made once per (V, dt) (launch_vturn).  The nearest 128th
+// / 2 pi, the exact product of V and dt / 2 pi (fx_vturn).  The nearest 128th
 // of a turn comes from a table of exp(2 pi i k / 128), the rest (at most
 // pi / 128) from the Taylor series, to 2^-58; one complex product joins the
 // two and one applies the result.  About 48 multiply-adds, where FP64 needs
 // some 70 operations at a 14th of their rate (the epilogue of the 256^3 z pass
 // 0.18 ms, the step of three passes 1.6 -> 1.2 ms; 128^2 step 42 -> 31 us).
 constexpr int FX_NL_TAB = 128;
-// The line-independent part of a call: beta dt / (2 pi) = (gh 2^32 + gl) 2^ge.
+// The line-independent part of a call: beta dt / (2 pi) = (gh 2^32 + gl) 2^ge,
+// dt / (2 pi) = d 2^de.
 struct FxNlArgs {
-    int gh, gl, ge;
-    const long long *vturn;  // V dt / (2 pi) per cell, 2^64 to a turn; nullable
-    const int *vbad;         // nonzero: V holds NaN or infinity; nullable
+    int gh, gl, ge, de;
+    long long d;
     const int4 *tab;         // exp(2 pi i k / 128), k < 128, as table constants
     const long long *tab2;   // 2^(k / 128) 2^61, k < 128 (imaginary time)
 };
@@ -362,6 +362,56 @@ __device__ __forceinline__ long long fx_theta(double rho, int gh, int gl, int ge
     const long long m = (long long)(((unsigned long long)mh << 32) | (unsigned long long)(lo << 10));
     const int sh = e ? e + ge - 957 : -63;  // 0 and denormals: 0
     return (fx_rmul(m, gh, gl) << min(max(sh, 0), 63)) >> min(max(-sh, 0), 63);
+}
+
+// 64-bit shifts whose amounts beyond 63 (negative ones, as unsigned, among them)
+// give 0
+__device__ __forceinline__ unsigned long long fx_shr(unsigned long long v, int s)
+{
+    asm("shr.b64 %0, %0, %1;" : "+l"(v) : "r"(s));
+    return v;
+}
+__device__ __forceinline__ unsigned long long fx_shl(unsigned long long v, int s)
+{
+    asm("shl.b64 %0, %0, %1;" : "+l"(v) : "r"(s));
+    return v;
+}
+__device__ __forceinline__ unsigned long long fx_madw_u(unsigned a, unsigned b, unsigned long long c)
+{
+    unsigned long long r;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+    return r;
+}
+// V d 2^de in 2^64ths of a turn (modulo one): the 53-bit significand of V times
+// |d| of at most 62 bits, exact, at the place of the exponents (denormals count
+// as 0).  *top keeps the largest exponent seen: 0x7ff for NaN and infinity, whose
+// angle means nothing.  A table of the products instead (one per time step, 8 bytes
+// per cell each) took memory that a field may not leave and was filled on the
+// first step after each change of V or dt.  Last pass with the flow, table -> here:
+// 64^2 4.5 -> 4.8 us, 128^2 5.5 -> 5.5, 256^2 6.0 -> 6.5, 128^3 63 -> 67, 256^3 496
+// -> 510, 240^3 765 -> 820; a new V, one step and the mass at 128^3 500 -> 404 us.
+__device__ __forceinline__ long long fx_vturn(double V, long long d, int de, int *top)
+{
+    const int hi = __double2hiint(V);
+    const unsigned lo = (unsigned)__double2loint(V);
+    const int e = (hi >> 20) & 0x7ff;
+    *top = max(*top, e);
+    const unsigned mh = (__funnelshift_l(lo, (unsigned)hi, 10) & 0x3fffffffu) | 0x40000000u, ml = lo << 10;
+    const unsigned long long md = (unsigned long long)(d < 0 ? -d : d);
+    const unsigned dh = (unsigned)(md >> 32), dl = (unsigned)md;
+    const unsigned long long p0 = fx_madw_u(ml, dl, 0);
+    const unsigned long long p1 = fx_madw_u(mh, dl, fx_madw_u(ml, dh, p0 >> 32));
+    const unsigned long long p2 = fx_madw_u(mh, dh, p1 >> 32);  // the product over 2^64
+    const int sh = e ? e + de - 957 : -64;
+    unsigned long long t = fx_shr(p2, -sh);
+    // an eighth of a turn and above: the product's lower half as well (a branch of
+    // the warp, which the compiler does not turn into selections)
+    if (__any_sync(__activemask(), sh > 0) && sh > 0) {
+        const unsigned long long pl = (p1 << 32) | (unsigned)p0;
+        t = fx_shl(p2, sh) | fx_shr(pl, 64 - sh) | fx_shl(pl, sh - 64);
+    }
+    const long long sg = (long long)((hi >> 31) ^ (int)(d >> 63));
+    return ((long long)t ^ sg) - sg;
 }
 
 // ---- 2^-x for FP64 x on the integer pipes (the flow of imaginary time) ----

@@ -381,11 +381,10 @@ void gpss_destroy(gpss_ctx *c)
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     clear_phases(c);  // and the graphs
-    clear_vturns(c);
     void *ptrs[] = {c->psi, c->scratch, c->V, c->tw[0], c->tw[1], c->tw[2], c->coord_dev[0],
                     c->coord_dev[1], c->coord_dev[2], c->partials, c->sums, c->scale, c->status,
                     c->counter, c->rk_buf[0], c->rk_buf[1], c->rk_buf[2], c->rk_buf[3], c->rk_lim,
-                    c->adj_buf, c->im_buf, c->tmap_dev, c->nl_tab, c->vbad};
+                    c->adj_buf, c->im_buf, c->tmap_dev, c->nl_tab};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     for (auto &e : c->ev)
@@ -552,8 +551,6 @@ int gpss_set_potential(gpss_ctx *c, const double *V)
     CUDA_TRY(c, cudaSetDevice(c->device));
     GPSS_TRY(flush_pending(c));
     clear_graphs(c);
-    clear_vturns(c);
-    if (c->vbad) CUDA_TRY(c, cudaMemsetAsync(c->vbad, 0, sizeof(int), c->stream));
     if (!V) { c->have_V = false; return GPSS_OK; }
     if (!c->V) GPSS_TRY(dev_alloc(c, &c->V, (size_t)c->total * real_bytes(c)));
     CUDA_TRY(c, cudaStreamSynchronize(c->stream));

@@ -316,8 +316,6 @@ inline bool reg_line(int64_t n) { return n >= 2 && n <= 256 && (n & (n - 1)) == 
 // pointwise kernels (pointwise.cu)
 cudaError_t launch_f64_to_f32(const double *in, float *out, int64_t count, cudaStream_t s);
 cudaError_t launch_f32_to_f64(const float *in, double *out, int64_t count, cudaStream_t s);
-cudaError_t launch_vturn(const double *V, long long *out, long long d, int de, int64_t count, int *bad,
-                         cudaStream_t s);
 template <typename T>
 cudaError_t launch_mul_phase(vec2<T> *data, const vec2<T> *phase, int64_t prow, int axis,
                              const int64_t *n, int64_t total, cudaStream_t s);

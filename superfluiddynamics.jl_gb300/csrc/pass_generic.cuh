@@ -464,8 +464,6 @@ gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
     const bool scaled = a.scale != nullptr;
     const T scale = scaled ? load_scale<T>(a.scale) : (T)1;
     const bool fxnl = MODE == MODE_FUSED && a.nl_mode == NL_REAL;
-    const bool vbad = MODE == MODE_FUSED && a.nl_fx.vbad && *a.nl_fx.vbad != 0;
-    (void)vbad;
     T acc_mass = 0, acc_pot = 0, acc_int = 0, acc_kin = 0, acc_rot = 0;
     double tot[RQ_COUNT] = {0.0, 0.0, 0.0, 0.0, 0.0};
 
@@ -655,18 +653,20 @@ gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
             (void)rsh;
             // 1/n: in the phase table, else here
             const bool byn = MODE == MODE_INV || mask;
-            const FxOut oc(qv, bad || vbad, byn ? (double)a.inv_n : 1.0, byn);
+            const FxOut oc(qv, bad, byn ? (double)a.inv_n : 1.0, byn);
             for (int i = i0; i < n; i += step) {
                 const uint32_t e = base + (uint32_t)i * st;
                 fxc u = data[at(i)];
                 u = fxc{u.y, u.x};
+                int vtop = 0;
                 if constexpr (MODE == MODE_FUSED) {
                     if (fxnl) {
-                        const long long vt = a.nl_fx.vturn && valid ? a.nl_fx.vturn[e] : 0;
+                        const long long vt = a.V && valid ? fx_vturn(a.V[e], a.nl_fx.d, a.nl_fx.de, &vtop) : 0;
                         u = fx_nl_real(u, vt, a.nl_fx.gh, a.nl_fx.gl, lsh, rsh, a.nl_fx.tab);
                     }
                 }
                 V v = oc(u, true);
+                if (vtop == 0x7ff) v.x = v.y = __longlong_as_double(0x7ff8000000000000LL);
                 if (!valid) continue;
                 if constexpr (MODE == MODE_FUSED) {
                     if (a.nl_mode != NL_NONE && !fxnl) {

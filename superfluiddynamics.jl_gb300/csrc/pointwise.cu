@@ -43,41 +43,6 @@ cudaError_t launch_f32_to_f64(const float *in, double *out, int64_t count, cudaS
     return cudaGetLastError();
 }
 
-// V dt / (2 pi) in 2^64ths of a turn (modulo one) for the fixed-point nonlinear
-// flow: the 53-bit significand of V times the 63-bit one of dt / (2 pi) = (dh
-// 2^32 + dl) 2^de, exact, at the position of the exponents.  *bad is set if any
-// V is not finite.
-__global__ void k_vturn(const double *__restrict__ V, long long *__restrict__ out, long long d, int de, int64_t count,
-                        int *__restrict__ bad)
-{
-    pdl_enter();
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const unsigned long long w = (unsigned long long)__double_as_longlong(V[i]);
-        const int e = (int)(w >> 52) & 0x7ff;
-        if (e == 0x7ff) *bad = 1;
-        const unsigned long long m = (w & 0xfffffffffffffULL) | (e ? 0x10000000000000ULL : 0);
-        const bool neg = ((w >> 63) != 0) != (d < 0);
-        const unsigned long long md = (unsigned long long)(d < 0 ? -d : d);
-        const unsigned long long hi = __umul64hi(m, md), lo = m * md;
-        const int sh = (e ? e : 1) - 1075 + de + 64;  // the product's unit in 2^-64 turns
-        unsigned long long t;
-        if (sh >= 64) t = 0;
-        else if (sh >= 0) t = lo << sh;
-        else if (sh > -64) t = (lo >> -sh) | (hi << (64 + sh));
-        else if (sh > -128) t = hi >> (-64 - sh);
-        else t = 0;
-        out[i] = (long long)(neg ? 0ULL - t : t);
-    }
-}
-
-cudaError_t launch_vturn(const double *V, long long *out, long long d, int de, int64_t count, int *bad,
-                         cudaStream_t s)
-{
-    launch_pdl(k_vturn, dim3(grid_for(count, 256)), dim3(256), 0, s, V, out, d, de, count, bad);
-    return cudaGetLastError();
-}
-
 // Plain form: psi_hat(k, row) *= phase(k, row) on a natural-order spectrum
 // along `axis` (the broadcasts of splitting.jl:167/172/190/195/200).  Table
 // rows are hi[n] then lo[n] (double-word factors); row `row` starts at row*prow.

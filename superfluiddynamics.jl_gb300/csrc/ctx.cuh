@@ -85,7 +85,9 @@ struct gpss_ctx {
     int *rk_lim = nullptr;    // RK: 2/3-rule limits per inner position (the FEAT_MASK pass)
     void *im_buf = nullptr;   // implicit schemes: work fields (implicit_impl)
     size_t im_bytes = 0;
-    int kry_hint = 0;         // iterations of the last Krylov solve (how many to issue at once)
+    // iterations of the Krylov solves of the last implicit step, by their place in it
+    // (how many to issue at once)
+    int kry_hint[16] = {0};
     // discrete adjoint: buffers kept between calls (sized for adj_nck checkpoints, adj_K states)
     void *adj_buf = nullptr;
     size_t adj_bytes = 0;

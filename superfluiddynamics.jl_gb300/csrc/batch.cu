@@ -589,7 +589,8 @@ static cudaError_t run_stacks(gpss_batch *b, int nsteps, double dt, double *mass
         };
         cudaError_t e = mass(0);
         if (e != cudaSuccess) return e;
-        const int wx = PassLauncher<float>::lines(n, true), wy = PassLauncher<float>::lines(n, false);
+        const int wx = PassLauncher<float>::lines(n, true, (int64_t)n * n),
+                  wy = PassLauncher<float>::lines(n, false, (int64_t)n * n);
         const int tiles_x = (n * P + wx - 1) / wx, tiles_y = (n * P + wy - 1) / wy;
         for (int s = 0; s <= nsteps; s++) {
             const int full = (s > 0 && s < nsteps) ? 1 : 0;

@@ -462,7 +462,7 @@ template <typename T> static int blocks_for(gpss_ctx *c, int axis)
                                      : std::min(1 << c->gplan32[axis].lw, c->gplan32[axis].W);
         return (int)((c->total / c->n[axis] + W - 1) / W);
     }
-    const int W = PassLauncher<T>::lines((int)c->n[axis], axis == 0);
+    const int W = PassLauncher<T>::lines((int)c->n[axis], axis == 0, c->total);
     const int64_t nl = c->total / c->n[axis];
     return (int)((nl + W - 1) / W);
 }

@@ -184,7 +184,7 @@ static int make_tensor_maps(gpss_ctx *c)
     const cuuint32_t estr[3] = {1, 1, 1};
     for (int axis = 1; axis <= 2; axis++) {
         const int64_t n = c->n[axis];
-        const int W = PassLauncher<float>::lines((int)n, false);
+        const int W = PassLauncher<float>::lines((int)n, false, c->total);
         if (n < 64 || W < 2 || c->n[0] % W) return GPSS_OK;
         const cuuint32_t box[3] = {(cuuint32_t)W, axis == 1 ? (cuuint32_t)n : 1u, axis == 2 ? (cuuint32_t)n : 1u};
         const CUresult r = reinterpret_cast<EncodeFn>(fn)(
@@ -504,8 +504,6 @@ int gpss_create(gpss_ctx **out, int ndim, const int64_t *n, const double *lo, co
         int b = precision == GPSS_FP32 ? blocks_for<float>(c, a) : blocks_for<double>(c, a);
         if (b > maxb) maxb = b;
     }
-    // (four cells per thread of 128: the FP64 passes of small fields)
-    if (precision == GPSS_FP64 && c->total <= QUAD_CELLS) maxb = std::max(maxb, (int)((c->total + 511) / 512));
     c->max_blocks = maxb;
     if ((rc = dev_alloc(c, (void **)&c->partials, sizeof(double) * RQ_COUNT * (size_t)maxb))) return bail(rc);
     if ((rc = dev_alloc(c, (void **)&c->sums, sizeof(double) * 4 * RQ_COUNT))) return bail(rc);

@@ -275,8 +275,9 @@ cudaError_t launch_pass_f32(int mode, bool xl, int n, const PassArgs<float> &a, 
                             cudaStream_t s);
 cudaError_t launch_pass_f64(int mode, bool xl, int n, const PassArgs<double> &a, int blocks,
                             cudaStream_t s);
-int pass_lines_per_cta_f32(int n, bool xl);
-int pass_lines_per_cta_f64(int n, bool xl);
+// lines of a CTA in the passes of a field of `total` cells
+int pass_lines_per_cta_f32(int n, bool xl, int64_t total);
+int pass_lines_per_cta_f64(int n, bool xl, int64_t total);
 // pipelined fused pass (FP32; n in {64, 128, 256}; tiles of 4096/n lines)
 cudaError_t launch_pipe_f32(bool xl, int n, const PassArgs<float> &a, int ntiles, cudaStream_t s);
 
@@ -288,7 +289,7 @@ template <typename T> struct PassLauncher;
 template <> struct PassLauncher<float> {
     static cudaError_t launch(int mode, bool xl, int n, const PassArgs<float> &a, int blocks,
                               cudaStream_t s) { return launch_pass_f32(mode, xl, n, a, blocks, s); }
-    static int lines(int n, bool xl) { return pass_lines_per_cta_f32(n, xl); }
+    static int lines(int n, bool xl, int64_t total) { return pass_lines_per_cta_f32(n, xl, total); }
     static cudaError_t pipe(bool xl, int n, const PassArgs<float> &a, int ntiles, cudaStream_t s)
     {
         return launch_pipe_f32(xl, n, a, ntiles, s);
@@ -301,7 +302,7 @@ template <> struct PassLauncher<float> {
 template <> struct PassLauncher<double> {
     static cudaError_t launch(int mode, bool xl, int n, const PassArgs<double> &a, int blocks,
                               cudaStream_t s) { return launch_pass_f64(mode, xl, n, a, blocks, s); }
-    static int lines(int n, bool xl) { return pass_lines_per_cta_f64(n, xl); }
+    static int lines(int n, bool xl, int64_t total) { return pass_lines_per_cta_f64(n, xl, total); }
     static cudaError_t pipe(bool, int, const PassArgs<double> &, int, cudaStream_t) { return cudaErrorInvalidValue; }
     static cudaError_t gen(int mode, const PassArgs<double> &a, const GenPlan &p, const Gen32Plan &, cudaStream_t s)
     {

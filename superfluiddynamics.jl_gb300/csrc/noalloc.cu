@@ -52,12 +52,17 @@ constexpr size_t kPartialBytes = GPSS_NOALLOC_SCRATCH_BYTES - kOffPartials;
 
 // The largest field the entry point takes (256^3) has at most 256^2 / W
 // tiles in one pass, W the lines of a CTA (fewest: 8), so its partial sums
-// need 8192 x 5 doubles = 320 KiB of the 969.5 KiB region (3x margin).  The run-time check below therefore never rejects a field of
-// lines up to 256; it guards the limit should the CTA shapes change.
+// need 8192 x 5 doubles = 320 KiB of the 969.5 KiB region (3x margin).  FP64
+// fields of up to QUAD_CELLS cells have CTAs of fewer lines (2 at 256 cells, 512
+// cells in all), which is 512 tiles at most.  The run-time check below therefore
+// never rejects a field of lines up to 256; it guards the limit should the CTA
+// shapes change.
 static_assert((uint64_t)(256 * 256 / PassShape<double, 256, true>::W) * RQ_COUNT * sizeof(double) <=
                   kPartialBytes, "the partial sums of a 256^3 FP64 field must fit the scratch array");
 static_assert((uint64_t)(256 * 256 / PassShape<double, 256, false>::W) * RQ_COUNT * sizeof(double) <=
                   kPartialBytes, "the partial sums of a 256^3 FP64 field must fit the scratch array");
+static_assert((uint64_t)(QUAD_CELLS / 256 / PassShape<double, 256, true, FEAT_SMALL>::W) * RQ_COUNT * sizeof(double) <=
+                  kPartialBytes, "the partial sums of a small FP64 field must fit the scratch array");
 
 std::mutex g_setup_mutex;
 unsigned char *g_scratch_dev[64] = {nullptr};  // looked-up device address, per device
@@ -149,7 +154,7 @@ int energy_noalloc_t(int ndim, const int64_t *n3, const double *lo, const double
         a.counter = counter;
         a.fin_out = sums + axis * RQ_COUNT;
         a.fin_mode = FIN_NONE;
-        const int W = PassLauncher<T>::lines((int)na, axis == 0);
+        const int W = PassLauncher<T>::lines((int)na, axis == 0, total);
         const int blocks = (int)((a.nlines + W - 1) / W);
         e = PassLauncher<T>::launch(MODE_DIAG, axis == 0, (int)na, a, blocks, stream);
         if (e != cudaSuccess) return noalloc_fail(GPSS_ECUDA, "diagnostic pass launch", e);
@@ -198,11 +203,12 @@ extern "C" int gpss_energy_noalloc(int ndim, const int64_t *n, const double *lo,
     // the partial sums of the largest pass must fit the fixed scratch, counted
     // from the tile count (an upper bound on the grid, which may be capped at
     // one wave).  The largest accepted field, 256^3 (CTAs of 8 lines: 8192
-    // tiles x 5 sums x 8 B = 320 KiB), fits with a 3x margin, so today this refusal is a guard for changed launch shapes.
+    // tiles x 5 sums x 8 B = 320 KiB), fits with a 3x margin, so today this
+    // refusal is a guard for changed launch shapes.
     const int64_t total = n3[0] * n3[1] * n3[2];
     for (int a = 0; a < ndim; a++) {
-        const int W = precision == GPSS_FP32 ? pass_lines_per_cta_f32((int)n3[a], a == 0)
-                                             : pass_lines_per_cta_f64((int)n3[a], a == 0);
+        const int W = precision == GPSS_FP32 ? pass_lines_per_cta_f32((int)n3[a], a == 0, total)
+                                             : pass_lines_per_cta_f64((int)n3[a], a == 0, total);
         const int64_t blocks = (total / n3[a] + W - 1) / W;
         if ((uint64_t)blocks * RQ_COUNT * sizeof(double) > kPartialBytes)
             return noalloc_fail(GPSS_EINVAL, "field too large for the fixed 1 MiB scratch of gpss_energy_noalloc");

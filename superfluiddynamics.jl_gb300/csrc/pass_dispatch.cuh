@@ -224,8 +224,13 @@ static cudaError_t launch_pipe_inst(const PassArgs<T> &a, int ntiles, cudaStream
     return cudaGetLastError();
 }
 
-template <typename T, int N> static int lines_per_cta_n(bool xl)
+// (the shape that launch_pass_mode takes for a field of `total` cells)
+template <typename T, int N> static int lines_per_cta_n(bool xl, int64_t total)
 {
+    if constexpr (quad_pass<T, N, FEAT_SMALL>) {
+        if (total <= QUAD_CELLS)
+            return xl ? PassShape<T, N, true, FEAT_SMALL>::W : PassShape<T, N, false, FEAT_SMALL>::W;
+    }
     return xl ? PassShape<T, N, true>::W : PassShape<T, N, false>::W;
 }
 
@@ -275,17 +280,17 @@ template <typename T, int N> static int lines_per_cta_n(bool xl)
         default: return cudaErrorInvalidValue;                                                 \
         }                                                                                      \
     }                                                                                          \
-    int pass_lines_per_cta_##SUFFIX(int n, bool xl)                                            \
+    int pass_lines_per_cta_##SUFFIX(int n, bool xl, int64_t total)                             \
     {                                                                                          \
         switch (n) {                                                                           \
-        case 2: return lines_per_cta_n<T, 2>(xl);                                              \
-        case 4: return lines_per_cta_n<T, 4>(xl);                                              \
-        case 8: return lines_per_cta_n<T, 8>(xl);                                              \
-        case 16: return lines_per_cta_n<T, 16>(xl);                                            \
-        case 32: return lines_per_cta_n<T, 32>(xl);                                            \
-        case 64: return lines_per_cta_n<T, 64>(xl);                                            \
-        case 128: return lines_per_cta_n<T, 128>(xl);                                          \
-        case 256: return lines_per_cta_n<T, 256>(xl);                                          \
+        case 2: return lines_per_cta_n<T, 2>(xl, total);                                       \
+        case 4: return lines_per_cta_n<T, 4>(xl, total);                                       \
+        case 8: return lines_per_cta_n<T, 8>(xl, total);                                       \
+        case 16: return lines_per_cta_n<T, 16>(xl, total);                                     \
+        case 32: return lines_per_cta_n<T, 32>(xl, total);                                     \
+        case 64: return lines_per_cta_n<T, 64>(xl, total);                                     \
+        case 128: return lines_per_cta_n<T, 128>(xl, total);                                   \
+        case 256: return lines_per_cta_n<T, 256>(xl, total);                                   \
         default: return 0;                                                                     \
         }                                                                                      \
     }

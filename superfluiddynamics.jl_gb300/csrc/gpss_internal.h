@@ -356,7 +356,7 @@ struct KrylovDev {
 };
 // what the dot products of a kernel are for (see implicit.cu)
 enum { KRY_NONE = 0, KRY_INIT = 1, KRY_ALPHA = 2, KRY_OMEGA = 3, KRY_CHECK = 4 };
-constexpr int KRY_MAX_CTAS = 304;  // of a kernel with dot products
+constexpr int KRY_MAX_CTAS = 152 * 8;  // of a kernel with dot products
 struct KryScratch {
     double *partials;        // [2 * KRY_MAX_CTAS]
     double *dots;            // the last two sums

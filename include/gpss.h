@@ -46,7 +46,8 @@ extern "C" {
                                  start of the call after each nonlinear stage */
 #define GPSS_FLAG_PIPE 8      /* x passes through the persistent asynchronous-copy
                                  pipeline (same arithmetic; the direct kernel is
-                                 faster on GB300 and is the default) */
+                                 faster on GB300 and is the default; FP64 contexts
+                                 run the direct kernel) */
 #define GPSS_FLAG_ENERGY_CACHE 16 /* real-time Strang (fused forms): every
                                  gpss_step also measures the energies of its
                                  final field in its last passes (with Omega != 0

@@ -24,8 +24,8 @@ struct DevBufs {
 };
 
 // one Strang step on `buf` as the forward of the adjoint: unmerged half
-// steps, no mass lock, so that the recomputed states are bitwise those of
-// the forward run
+// steps, no mass lock, so that the recomputed states are those of the forward
+// run (bitwise: the recompute repeats its launches)
 template <typename T> static int strang_on(gpss_ctx *c, void *buf, double dt)
 {
     GPSS_TRY(kinetic_fused<T>(c, dt * 0.5, 0, true, dt, 0, false, false, FIN_NONE, buf));
@@ -74,7 +74,9 @@ static int adj_group(gpss_ctx *c, void *buf, double dtl, bool reverse, bool nl, 
 //   dL/dpsi0 = L^H(h) g
 // one group per step with N^H fused into its last pass.  Segments of K steps
 // are recomputed from their checkpoint into K state buffers (the same
-// kernels as the forward, so the states are bitwise the forward's).  The
+// kernels as the forward after one nonlinear sweep of the checkpoint: bitwise the
+// forward's states in FP32; in FP64 to rounding, because the forward's flow
+// takes the pass's integers and the sweep the state rounded to FP64).  The
 // recompute of segment s-1 runs on a second stream while the backward sweep
 // works through segment s (two sets of state buffers, alternating): a 256^2
 // pass fills a few dozen SMs, so the two chains share the GPU.

@@ -1,7 +1,7 @@
 // fft_fix.cuh -- FP64 fields transformed in 64-bit fixed point.
 //
-// GB300 runs FP64 at 2 operations per clock and SM, 32-bit integer additions at
-// 128 and 32x32 -> 64-bit multiply-adds at ~24 (measured).  A transform in
+// GB300 runs FP64 at 1.7 operations per clock and SM, 32-bit integer additions at
+// 119 and 32x32 -> 64-bit multiply-adds at ~24 (measured).  A transform in
 // FP64 arithmetic is bound by that pipe alone (72 operations per cell and
 // pass of 256-cell lines: 2.5 ms at 256^3, against 0.08 ms of memory traffic),
 // so the passes of FP64 fields hold the values of a line as 64-bit integers
@@ -241,7 +241,8 @@ __device__ __forceinline__ long long fx_from(double x, int s0)
     return ((((long long)(m >> s)) ^ sg) - sg + 1) >> 1;
 }
 
-// v 2^q in FP64 by integer operations, |q| <= 900
+// v 2^q in FP64 by integer operations, |q| <= 900, rounded to nearest (halves away
+// from zero)
 __device__ __forceinline__ double fx_double(long long v, int q)
 {
     const int sg = (int)(v >> 63);
@@ -265,9 +266,10 @@ __device__ __forceinline__ double fx_double(long long v, int q)
 // / 2 pi, the exact product of V and dt / 2 pi (fx_vturn).  The nearest 128th
 // of a turn comes from a table of exp(2 pi i k / 128), the rest (at most
 // pi / 128) from the Taylor series, to 2^-58; one complex product joins the
-// two and one applies the result.  About 48 multiply-adds, where FP64 needs
-// some 70 operations at a 14th of their rate (the epilogue of the 256^3 z pass
-// 0.18 ms, the step of three passes 1.6 -> 1.2 ms; 128^2 step 42 -> 31 us).
+// two and one applies the result.  About 48 multiply-adds, 4 more with a
+// potential, where FP64 needs some 70 operations at a 14th of their rate (the
+// epilogue of the 256^3 z pass 0.20 ms, 0.22 with a potential, where FP64 took
+// 0.6 more).
 constexpr int FX_NL_TAB = 128;
 // The line-independent part of a call: beta dt / (2 pi) = (gh 2^32 + gl) 2^ge,
 // dt / (2 pi) = d 2^de.
@@ -418,7 +420,8 @@ __device__ __forceinline__ long long fx_vturn(double V, long long d, int de, int
 //
 // -x as a 52-bit fraction below an 11-bit integer; the nearest 128th from a
 // table, the rest r (at most 1/256) from the series of 2^r to 2^-60, the integer
-// as the exponent: an FP64 value off by its last rounding and the 2^-53 of x's.
+// as the exponent: an FP64 value off by its last rounding and the 2^-53 of x's,
+// and 0 below 2^-1022 (a pass has no quantum for subnormal values).
 // 17 multiply-adds, where FP64 exp is some 20 operations at a 14th of their
 // rate (128^3 imaginary-time x pass 151 -> 92 us).
 constexpr long long FX_E1 = 0x2c5c85fdf473de7LL, FX_E2 = 0x3d7f7bff058b2LL, FX_E3 = 0x38d611ae094LL, FX_E4 = 0x276556df7LL;

@@ -168,8 +168,8 @@ __device__ __forceinline__ float nl_theta_bound(float rmax, float vmax, const NL
 
 // The factor f = exp(-i theta) (real time) or exp(-theta) (imaginary time,
 // returned as (f, 0)) of one cell; the step is psi <- f psi (nl_rotate).  The
-// discrete adjoint recomputes the same factor, so forward and backward agree
-// to the bit.
+// discrete adjoint of FP32 fields recomputes the same factor, so forward and
+// backward agree to the bit (FP64: to rounding, see fx_nl_real and fx_theta).
 __device__ __forceinline__ double2 nl_factor(double2 v, double Vv, const NLConst<double> &c, bool imag)
 {
     const double rho = v.x * v.x + v.y * v.y;          // abs2

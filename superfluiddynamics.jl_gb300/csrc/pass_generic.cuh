@@ -169,7 +169,7 @@ inline int gen_mode_at(const GenPlan &p, int pos)
 // four tiles per SM) -- and the W that makes that product smallest is taken, at
 // least 4 adjacent columns for strided lines (32 or 64 contiguous bytes) and
 // at most 44 KB of tile (four per SM, with their tables).  The product itself
-// goes to *time.
+// goes to *time.  (152 SMs: those of a GB300, whose measurements these are.)
 inline int gen_tile_log(int n, const int *radix, int nst, int64_t nlines, bool xl, int most, double *time = nullptr)
 {
     const int low = xl ? 0 : 2;

@@ -14,7 +14,9 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libgpss.so")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
+# (device code uncompressed: nvcc compresses a unit's code above about 10 MB, and the first
+# kernel of such a unit then waits 10 to 13 ms for it to be unpacked)
+NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "--no-compress", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
               "-I" + os.path.join(HERE, "..", "include")]
 
 

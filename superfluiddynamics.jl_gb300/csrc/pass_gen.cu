@@ -41,12 +41,12 @@ cudaError_t gen_launch_kernel(void (*k)(const PassArgs<T>, const P), int threads
 // cells of a tile of x lines (padded) or columns
 size_t gen_slots(int n, int W, bool xl) { return (size_t)W * (size_t)(xl ? n + (n >> 4) + 1 : n); }
 
-template <int MODE, int KIND = GEN_PLAIN> cudaError_t gen_launch_f64(const PassArgs<double> &a, const GenPlan &p, cudaStream_t s)
+template <int MODE, bool MULT = false> cudaError_t gen_launch_f64(const PassArgs<double> &a, const GenPlan &p, cudaStream_t s)
 {
     const int W = p.lines();
     const bool phase = MODE == MODE_FUSED && a.prow == 0 && !a.mask_lim;
     const size_t smem = 16 * ((size_t)(phase ? 2 * p.n : p.n) + gen_slots(p.n, W, a.stride == 1));
-    return gen_launch_kernel(gen_pass_kernel<MODE, KIND>, GEN_THREADS, smem, (a.nlines + W - 1) / W, a, p, s);
+    return gen_launch_kernel(gen_pass_kernel<MODE, MULT>, GEN_THREADS, smem, (a.nlines + W - 1) / W, a, p, s);
 }
 
 template <int MODE> cudaError_t gen_launch_f32(const PassArgs<float> &a, const Gen32Plan &p, cudaStream_t s)
@@ -92,9 +92,8 @@ cudaError_t launch_gen_f64(int mode, const PassArgs<double> &a, const GenPlan &p
     switch (mode) {
     case MODE_FUSED:
         if (!a.phase && !a.mask_lim) return cudaErrorInvalidValue;
-        if (a.mult && (a.mask_lim || a.nl_pre || a.nl_mode == NL_REAL)) return cudaErrorInvalidValue;
-        if (a.mult) return gen_launch_f64<MODE_FUSED, GEN_MULT>(a, p, s);
-        if (a.nl_mode == NL_REAL) return gen_launch_f64<MODE_FUSED, GEN_FLOW>(a, p, s);
+        if (a.mult && (a.mask_lim || a.nl_pre)) return cudaErrorInvalidValue;
+        if (a.mult) return gen_launch_f64<MODE_FUSED, true>(a, p, s);
         return gen_launch_f64<MODE_FUSED>(a, p, s);
     case MODE_FWD: return gen_launch_f64<MODE_FWD>(a, p, s);
     case MODE_INV: return gen_launch_f64<MODE_INV>(a, p, s);

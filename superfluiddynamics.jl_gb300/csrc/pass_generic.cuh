@@ -413,10 +413,8 @@ __device__ __noinline__ void gen_stage_loop(const GenPlan &p, int s, int kind, i
     }
 }
 
-// GEN_FLOW: with the nonlinear flow of real time; GEN_MULT: the phase is a
-// multiplier table (fft_fix.cuh)
-enum { GEN_PLAIN = 0, GEN_FLOW = 1, GEN_MULT = 2 };
-template <int MODE, int KIND = GEN_PLAIN>
+// MULT: the phase is a multiplier table (fft_fix.cuh)
+template <int MODE, bool MULT = false>
 __global__ void __launch_bounds__(GEN_THREADS, 4)
 gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
 {
@@ -432,8 +430,7 @@ gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
     const bool rowph = MODE == MODE_FUSED && a.prow != 0;
     const bool mask = MODE == MODE_FUSED && a.mask_lim != nullptr;
     fxc *data = reinterpret_cast<fxc *>(sph + (MODE == MODE_FUSED && !rowph && !mask ? n : 0));
-    constexpr bool MULT = KIND == GEN_MULT, fxnl = KIND == GEN_FLOW;
-    static_assert(KIND == GEN_PLAIN || MODE == MODE_FUSED, "the flow and multipliers: fused passes");
+    static_assert(!MULT || MODE == MODE_FUSED, "multipliers: fused passes");
     __shared__ int sword[64], smword[64];    // (m: of the multiplied spectrum)
     __shared__ unsigned ssum[64], smsum[64];
     const int tid = threadIdx.x;
@@ -466,6 +463,7 @@ gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const bool scaled = a.scale != nullptr;
     const T scale = scaled ? load_scale<T>(a.scale) : (T)1;
+    const bool fxnl = MODE == MODE_FUSED && a.nl_mode == NL_REAL;
     T acc_mass = 0, acc_pot = 0, acc_int = 0, acc_kin = 0, acc_rot = 0;
     double tot[RQ_COUNT] = {0.0, 0.0, 0.0, 0.0, 0.0};
 
@@ -656,26 +654,22 @@ gen_pass_kernel(const PassArgs<double> a, const __grid_constant__ GenPlan p)
             // 1/n: in the phase table, else here
             const bool byn = MODE == MODE_INV || mask;
             const FxOut oc(qv, bad, byn ? (double)a.inv_n : 1.0, byn);
-            // (the flow's potential is read one cell ahead)
-            const bool withv = fxnl && a.V && valid;
-            T vnext = withv && i0 < n ? a.V[base + (uint32_t)i0 * st] : (T)0;
-            (void)vnext;
             for (int i = i0; i < n; i += step) {
                 const uint32_t e = base + (uint32_t)i * st;
                 fxc u = data[at(i)];
                 u = fxc{u.y, u.x};
                 int vtop = 0;
-                if constexpr (fxnl) {
-                    const T vcell = vnext;
-                    if (withv && i + step < n) vnext = a.V[e + (uint32_t)step * st];
-                    const long long vt = withv ? fx_vturn(vcell, a.nl_fx.d, a.nl_fx.de, &vtop) : 0;
-                    u = fx_nl_real(u, vt, a.nl_fx.gh, a.nl_fx.gl, lsh, rsh, a.nl_fx.tab);
+                if constexpr (MODE == MODE_FUSED) {
+                    if (fxnl) {
+                        const long long vt = a.V && valid ? fx_vturn(a.V[e], a.nl_fx.d, a.nl_fx.de, &vtop) : 0;
+                        u = fx_nl_real(u, vt, a.nl_fx.gh, a.nl_fx.gl, lsh, rsh, a.nl_fx.tab);
+                    }
                 }
                 V v = oc(u, true);
                 if (vtop == 0x7ff) v.x = v.y = __longlong_as_double(0x7ff8000000000000LL);
                 if (!valid) continue;
                 if constexpr (MODE == MODE_FUSED) {
-                    if (!fxnl && a.nl_mode != NL_NONE) {
+                    if (a.nl_mode != NL_NONE && !fxnl) {
                         v = NLImag64(a.nl_beta, a.nl_dt, 1.0, a.nl_fx.tab2)(v, a.V ? a.V[e] : (T)0);  // imaginary time
                     }
                     if (red & RED_POINT) {
